@@ -106,14 +106,13 @@ __device__ __forceinline__ void model_pair(const float* c11, const float* c13, c
 // Producer side of one item: TMA loads of every plane of the item's range.
 __device__ __forceinline__ bool fwd_produce(const FwdCommon& a, const FwdMaps& m, int* status,
                                             int li, unsigned char* smem, uint64_t* full,
-                                            uint64_t* empty, long long& k) {
+                                            uint64_t* empty, RingPos<F_STAGES>& k) {
   int bx, by, z0, z1;
   item(a.sc, li, bx, by, z0, z1);
   const int x0 = bx * TX, y0 = kHalo + by * TY;
-  for (int z = z0; z < z1; ++z, ++k) {
-    const int s = (int)(k % F_STAGES);
-    if (k >= F_STAGES && !mbar_wait(&empty[s], (uint32_t)(((k / F_STAGES) & 1) ^ 1), status))
-      return false;
+  for (int z = z0; z < z1; ++z, k.advance()) {
+    const int s = k.s;
+    if (!mbar_wait(&empty[s], k.ph ^ 1u, status)) return false;
     const int zp = z + kZPad;
     unsigned char* st = smem + s * F_STAGE_BYTES;
     mbar_arrive_expect_tx(&full[s], F_STAGE_BYTES);
@@ -136,7 +135,7 @@ template <bool kProbe, bool kExact = false>
 __device__ __forceinline__ bool fwd_consume(const FwdCommon& a, const FwdPar& bp,
                                             const Probe& probe, int* status, int li, float amp,
                                             const unsigned char* smem, uint64_t* full,
-                                            uint64_t* empty, long long& k, int warp, int lane) {
+                                            uint64_t* empty, RingPos<F_STAGES>& k, int warp, int lane) {
   const bool damp = a.dampz != nullptr;
   const int ry = warp * 2 + (lane >> 4);
   const int xo = 2 * (lane & 15);
@@ -179,7 +178,7 @@ __device__ __forceinline__ bool fwd_consume(const FwdCommon& a, const FwdPar& bp
 #pragma unroll
   for (int j = 0; j < 4; ++j) dzr[j] = (damp && z0 - 4 + j >= 0) ? a.dampz[z0 - 4 + j] : 1.f;
   float dz_next = damp ? a.dampz[z0] : 1.f;
-  for (int z = z0; z < z1; ++z, ++k) {
+  for (int z = z0; z < z1; ++z, k.advance()) {
     const float dz = dz_next;
     if (damp && z + 1 < z1) dz_next = a.dampz[z + 1];
 #pragma unroll
@@ -188,8 +187,8 @@ __device__ __forceinline__ bool fwd_consume(const FwdCommon& a, const FwdPar& bp
     // the model pair: loads issued before the stage wait
     float2 c11, c13, c33;
     model_pair(a.c11, a.c13, a.c33, (long long)z * a.d.plane + off, v0 || v1, c11, c13, c33);
-    const int s = (int)(k % F_STAGES);
-    if (!mbar_wait(&full[s], (uint32_t)((k / F_STAGES) & 1), status)) return false;
+    const int s = k.s;
+    if (!mbar_wait(&full[s], k.ph, status)) return false;
     const unsigned char* st = smem + s * F_STAGE_BYTES;
     const float* sh = (const float*)(st + F_OFF_H) + sr;
     const float* pl = (const float*)(st + F_OFF_Z) + pi;  // [z+4][prev x][prev z]
@@ -313,7 +312,7 @@ __global__ void __launch_bounds__(NTHREADS, 3)
   uint64_t *full, *empty;
   unsigned char* smem = ring_init<F_STAGES, F_STAGE_BYTES>(smem_raw, full, empty);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  long long k = 0;  // planes issued / consumed by this CTA
+  RingPos<F_STAGES> k;  // planes issued / consumed by this CTA
   if (warp == NCW) {  // ---------------- producer
     if (lane == 0)
       for (int it = blockIdx.x; it < a0.c.sc.items; it += gridDim.x)
@@ -360,7 +359,7 @@ __global__ void __launch_bounds__(NTHREADS, 3) k_fwd3d_batch(const __grid_consta
   uint64_t *full, *empty;
   unsigned char* smem = ring_init<F_STAGES, F_STAGE_BYTES>(smem_raw, full, empty);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  long long k = 0;
+  RingPos<F_STAGES> k;
   if (warp == NCW) {
     if (lane == 0)
       for (int it = blockIdx.x; it < B.items; it += gridDim.x) {
@@ -439,14 +438,13 @@ constexpr float kTwoThirdF = (float)kTwoThird, kOneThirdF = (float)kOneThird;
 template <bool kRtm>
 __device__ __forceinline__ bool bwd_produce(const BwdCommon& a, const BwdMaps& m, int* status,
                                             int li, unsigned char* smem, uint64_t* full,
-                                            uint64_t* empty, long long& k) {
+                                            uint64_t* empty, RingPos<B_STAGES>& k) {
   int bx, by, z0, z1;
   item(a.sc, li, bx, by, z0, z1);
   const int x0 = bx * TX, y0 = kHalo + by * TY;
-  for (int z = z0; z < z1; ++z, ++k) {
-    const int s = (int)(k % B_STAGES);
-    if (k >= B_STAGES && !mbar_wait(&empty[s], (uint32_t)(((k / B_STAGES) & 1) ^ 1), status))
-      return false;
+  for (int z = z0; z < z1; ++z, k.advance()) {
+    const int s = k.s;
+    if (!mbar_wait(&empty[s], k.ph ^ 1u, status)) return false;
     const int zp = z + kZPad;
     unsigned char* st = smem + s * B_STAGE_BYTES;
     unsigned char* pl = st + B_OFF_P;
@@ -467,7 +465,7 @@ __device__ __forceinline__ bool bwd_produce(const BwdCommon& a, const BwdMaps& m
 template <bool kRtm>
 __device__ __forceinline__ bool bwd_consume(const BwdCommon& a, const BwdPar& bp, int* status,
                                             int li, float amp, const unsigned char* smem,
-                                            uint64_t* full, uint64_t* empty, long long& k,
+                                            uint64_t* full, uint64_t* empty, RingPos<B_STAGES>& k,
                                             int warp, int lane) {
   const int ry = warp * 2 + (lane >> 4);
   const int xo = 2 * (lane & 15);
@@ -516,7 +514,7 @@ __device__ __forceinline__ bool bwd_consume(const BwdCommon& a, const BwdPar& bp
     r13 = (anyv && !kRtm) ? __ldg(reinterpret_cast<const float2*>(a.g13 + i)) : zero;
     r33 = (anyv && !kRtm) ? __ldg(reinterpret_cast<const float2*>(a.g33 + i)) : zero;
   };
-  for (int z = z0; z < z1; ++z, ++k) {
+  for (int z = z0; z < z1; ++z, k.advance()) {
     const float dz = dz_next;
     if (z + 1 < z1) dz_next = a.dampz[z + 1];
     // issued before the stage wait: the loads complete while the stage
@@ -527,8 +525,8 @@ __device__ __forceinline__ bool bwd_consume(const BwdCommon& a, const BwdPar& bp
 #pragma unroll
     for (int j = 0; j < 3; ++j) dzr[j] = dzr[j + 1];
     dzr[3] = dz;
-    const int s = (int)(k % B_STAGES);
-    if (!mbar_wait(&full[s], (uint32_t)((k / B_STAGES) & 1), status)) return false;
+    const int s = k.s;
+    if (!mbar_wait(&full[s], k.ph, status)) return false;
     const unsigned char* st = smem + s * B_STAGE_BYTES;
     const float* sh = (const float*)(st + B_OFF_SH) + sr;
     const float* lh = (const float*)(st + B_OFF_LH) + sr;
@@ -647,7 +645,7 @@ __global__ void __launch_bounds__(NTHREADS, 2)
   uint64_t *full, *empty;
   unsigned char* smem = ring_init<B_STAGES, B_STAGE_BYTES>(smem_raw, full, empty);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  long long k = 0;
+  RingPos<B_STAGES> k;
   if (warp == NCW) {
     if (lane == 0)
       for (int it = blockIdx.x; it < a0.c.sc.items; it += gridDim.x)
@@ -674,7 +672,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_bwd3d_batch(const __grid_consta
   uint64_t *full, *empty;
   unsigned char* smem = ring_init<B_STAGES, B_STAGE_BYTES>(smem_raw, full, empty);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  long long k = 0;
+  RingPos<B_STAGES> k;
   if (warp == NCW) {
     if (lane == 0)
       for (int it = blockIdx.x; it < B.items; it += gridDim.x) {
