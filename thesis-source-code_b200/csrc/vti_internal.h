@@ -190,12 +190,14 @@ int make_tile_maps_typed(vti_ctx* ctx, const Dims3& d, void* alloc, int elem_byt
 // all z): next written through px_ptr/pz_ptr (prev is read through the px/pz
 // maps; the same volume for an in-place step); damp == nullptr: no sponge
 // (random-boundary pass); exact: the sponge as a plain diagonal (exact-mode
-// operator). TMA-pipelined, see vti_tma3d.cu.
+// operator). up: march the volume from its last plane to its first (a time
+// loop alternates the directions, see vti_tma3d.cu).
 int launch_fwd3d_tma(vti_ctx* ctx, const Dims3& d, const TileMaps& cx, const TileMaps& cz,
                      const TileMaps& px, const TileMaps& pz, const TileMaps& c11,
                      const TileMaps& c13, const TileMaps& c33, const float* cz_ptr,
                      float* px_ptr, float* pz_ptr, const Damping* damp, float sx, float sy,
-                     float sz, PointSource src, Probe probe = Probe(), bool exact = false);
+                     float sz, PointSource src, Probe probe = Probe(), bool exact = false,
+                     bool up = false);
 // Fused backward step: sigma back one level (gradient form, no sponge, +src),
 // adjoint lambda one level (forward form, sponge), zero-lag imaging into g
 // (rtm: the RTM image in g11 instead).
@@ -207,7 +209,7 @@ int launch_bwd3d_tma(vti_ctx* ctx, const Dims3& d, const TileMaps& scx, const Ti
                      const float* scz_ptr, const float* lcz_ptr, float* spx_ptr, float* spz_ptr,
                      float* lpx_ptr, float* lpz_ptr, float* g11_ptr, float* g13_ptr,
                      float* g33_ptr, const Damping& damp, float dt2, float idx2, float idy2,
-                     float idz2, float sx, float sy, float sz, PointSource src, bool rtm);
+                     float idz2, float sx, float sy, float sz, PointSource src, bool rtm, bool up = false);
 
 // One job of a batched forward launch (k_fwd3d_tma over the items of many
 // volumes). Step s = tick - t0 of the job uses parity p = s & 1:

@@ -222,7 +222,7 @@ int fwd_level(vti3d_plan* p, const ShotGeom& s, bool sponge, int A, int B, int i
   VTI_TRY(launch_fwd3d_tma(ctx, p->d, p->m_sx[A], p->m_sz[A], p->m_sx[B], p->m_sz[B], cm[0],
                            cm[1], cm[2], p->sz[A].origin, p->sx[B].origin, p->sz[B].origin,
                            sponge ? &dmp : nullptr, dt2 / (g.dx * g.dx), dt2 / (g.dy * g.dy),
-                           dt2 / (g.dz * g.dz), src));
+                           dt2 / (g.dz * g.dz), src, Probe(), false, (it & 1) != 0));
   if (sponge && it < (int)s.rec_at.size() && s.rec_at[it] >= 0)
     VTI_TRY(launch_record(ctx, p->d_trace, nnt_of(g), s.rec_at[it], p->sx[B].origin,
                           p->sz[B].origin, p->d_rec, s.nr));
@@ -285,7 +285,8 @@ int bwd_level(vti3d_plan* p, const ShotGeom& s, bool rtm, int SA, int SB, int LA
       p->m_lx[LB], p->m_lz[LB], cm[0], cm[1], cm[2], p->m_g[0], p->m_g[1], p->m_g[2],
       p->sz[SA].origin, p->lz[LA].origin, p->sx[SB].origin, p->sz[SB].origin,
       p->lx[LB].origin, p->lz[LB].origin, p->g11.origin, p->g13.origin, p->g33.origin, dmp,
-      dt2, 1.f / dx2, 1.f / dy2, 1.f / dz2, dt2 / dx2, dt2 / dy2, dt2 / dz2, src, rtm));
+      dt2, 1.f / dx2, 1.f / dy2, 1.f / dz2, dt2 / dx2, dt2 / dy2, dt2 / dz2, src, rtm,
+      (i & 1) != 0));
   // residual interpolated at it+1 (injectRecord3d.cu:60-78)
   const int ti = it + 1;
   float f = float(ti) / float(st);
@@ -850,7 +851,7 @@ int vti3d_plan_wavelet_gradient(vti3d_plan* p, const float* souloc, const int* s
       VTI_TRY(launch_fwd3d_tma(ctx, d, p->m_lx[LA], p->m_lz[LA], p->m_lx[LB], p->m_lz[LB],
                                p->m_cpad[0], p->m_cpad[1], p->m_cpad[2], p->lz[LA].origin,
                                p->lx[LB].origin, p->lz[LB].origin, &dmp, sxs, sys, szs,
-                               PointSource(), probe));
+                               PointSource(), probe, false, (i & 1) != 0));
       const int ti = it + 1;
       float f = float(ti) / float(st);
       int i0 = (int)f;

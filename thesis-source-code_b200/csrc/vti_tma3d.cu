@@ -103,21 +103,84 @@ __device__ __forceinline__ void model_pair(const float* c11, const float* c13, c
   a33 = any ? __ldg(reinterpret_cast<const float2*>(c33 + i)) : zero;
 }
 
+// March direction. kDir = 1 walks every item down z as numbered; kDir = -1
+// walks the items in reverse order and each item from its last plane to its
+// first. A time loop alternates the two, so a level starts on the planes the
+// level before it touched last, while they are still in L2 (126 MB): a level
+// that always starts at plane 0 finds nothing of a volume set larger than L2
+// there. Every point is computed by the same operations in either direction.
+// Measured, one direction -> alternating (nt 400): gradient 251x203x150 94.6 ->
+// 89.2 ms, 400x400x200 360 -> 350 ms, RTM 256x224x128 61.1 -> 56.5 ms; no
+// change where a level's volumes fit L2 (128^3 modeling 15.5 ms).
+template <int kDir>
+__device__ __forceinline__ int march_item(int i, int items) {
+  return kDir > 0 ? i : items - 1 - i;
+}
+
+// z queue of one x pair: q[j] holds plane z - 4 + j; `in` is plane z + 4
+// (kDir > 0) or z - 4. (Nine unrolled copies of the plane loop with rotating
+// slots save the moves but spill: 482 ms per 400x400x200 gradient of 399
+// levels against 350.)
+template <int kDir>
+__device__ __forceinline__ void queue_shift(float2 (&q)[9], float2 in) {
+  if (kDir > 0) {
+#pragma unroll
+    for (int kk = 0; kk < 8; ++kk) q[kk] = q[kk + 1];
+    q[8] = in;
+  } else {
+#pragma unroll
+    for (int kk = 8; kk > 0; --kk) q[kk] = q[kk - 1];
+    q[0] = in;
+  }
+}
+
+// The sponge's block order (abc3d.cu:82-126): the z stencil reads the planes of
+// the 4-plane blocks above its own already damped. Marching down z, the queue
+// entries of a block are damped once, after its last plane (z; entries 1..4 are
+// planes z-3 .. z then). dampz is read from L1 (one line, the same address for
+// all threads).
+__device__ __forceinline__ void damp_finished_block(float2 (&q)[9], const float (&dxy)[2],
+                                                    const float* dampz, int z, int nz) {
+  if (((z + 1) & 3) == 0 && z + 1 < nz) {
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      const float d = __ldg(dampz + z - 3 + kk);
+      q[kk + 1] = mul2(q[kk + 1], make_float2(dxy[0] * d, dxy[1] * d));
+    }
+  }
+}
+// Marching up, the queue keeps the stored values (a plane above is read damped
+// by this block and undamped by its own later): u[j] = plane z - 4 + j lies in
+// a block above iff j < 4 - z % 4 (planes above the volume hold zeros).
+__device__ __forceinline__ void damp_above(float2 (&u)[4], const float (&dxy)[2],
+                                           const float* dampz, int z) {
+  const int m = z < 4 ? 0 : 4 - (z & 3);
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if (j < m) {
+      const float d = __ldg(dampz + z - 4 + j);
+      u[j] = mul2(u[j], make_float2(dxy[0] * d, dxy[1] * d));
+    }
+}
+
 // Producer side of one item: TMA loads of every plane of the item's range.
+template <int kDir>
 __device__ __forceinline__ bool fwd_produce(const FwdCommon& a, const FwdMaps& m, int* status,
                                             int li, unsigned char* smem, uint64_t* full,
                                             uint64_t* empty, RingPos<F_STAGES>& k) {
   int bx, by, z0, z1;
   item(a.sc, li, bx, by, z0, z1);
   const int x0 = bx * TX, y0 = kHalo + by * TY;
-  for (int z = z0; z < z1; ++z, k.advance()) {
+  const int nz = z1 - z0;
+  for (int n = 0; n < nz; ++n, k.advance()) {
+    const int z = kDir > 0 ? z0 + n : z1 - 1 - n;
     const int s = k.s;
     if (!mbar_wait(&empty[s], k.ph ^ 1u, status)) return false;
     const int zp = z + kZPad;
     unsigned char* st = smem + s * F_STAGE_BYTES;
     mbar_arrive_expect_tx(&full[s], F_STAGE_BYTES);
     tma_load(st + F_OFF_H, &m.cx, &full[s], x0 - kHalo, y0 - kHalo, zp);
-    tma_load(st + F_OFF_Z, &m.cz, &full[s], x0, y0, zp + kHalo);
+    tma_load(st + F_OFF_Z, &m.cz, &full[s], x0, y0, zp + kDir * kHalo);
     tma_load(st + F_OFF_PX, &m.px, &full[s], x0, y0, zp);
     tma_load(st + F_OFF_PZ, &m.pz, &full[s], x0, y0, zp);
   }
@@ -131,17 +194,19 @@ __device__ __forceinline__ bool fwd_produce(const FwdCommon& a, const FwdMaps& m
 // Gauss-Newton product uses: centred damping next = D (C L cur + 2 cur + src)
 // - (2D - 1) prev (energy-stable for D <= 1), no block-order reading of the
 // z stencil.
-template <bool kProbe, bool kExact = false>
+// kSponge: the sponge on, off, or (batched jobs) on where the job has tables.
+enum SpongeMode { kSpongeOff = 0, kSpongeOn = 1, kSpongeByJob = 2 };
+template <bool kProbe, bool kExact, int kDir, int kSponge>
 __device__ __forceinline__ bool fwd_consume(const FwdCommon& a, const FwdPar& bp,
                                             const Probe& probe, int* status, int li, float amp,
                                             const unsigned char* smem, uint64_t* full,
                                             uint64_t* empty, RingPos<F_STAGES>& k, int warp, int lane) {
-  const bool damp = a.dampz != nullptr;
+  const bool damp = kSponge == kSpongeByJob ? a.dampz != nullptr : kSponge == kSpongeOn;
   const int ry = warp * 2 + (lane >> 4);
   const int xo = 2 * (lane & 15);
   const int sr = (ry + kHalo) * HX + xo + kHalo;  // centre in the halo tile
   const int pi = ry * TX + xo;                    // centre in a plain tile
-  float2 q[9];  // z queue of the pair: planes z-4 .. z+4
+  float2 q[9];  // z queue of the pair
   float dxy[2];
   int bx, by, z0, z1;
   item(a.sc, li, bx, by, z0, z1);
@@ -156,46 +221,38 @@ __device__ __forceinline__ bool fwd_consume(const FwdCommon& a, const FwdPar& bp
   const int prb_e = (kProbe && y == probe.y && probe.x >= 0) ? probe.x - x : -1;
   dxy[0] = (damp && v0) ? a.dampx[x] * a.dampy[y] : 1.f;
   dxy[1] = (damp && v1) ? a.dampx[x + 1] * a.dampy[y] : 1.f;
-  // start the queue: planes z0-4 .. z0+3 from global
-  q[0] = make_float2(0.f, 0.f);
+  // start the queue from global, one shift before the first plane: planes
+  // z0-4 .. z0+3 in q[1..8] (marching down the array: z1-4 .. z1+3 in q[0..7])
+  q[kDir > 0 ? 0 : 8] = make_float2(0.f, 0.f);
 #pragma unroll
-  for (int kk = 1; kk < 9; ++kk) {
-    const int zz = z0 - 5 + kk;
+  for (int kk = kDir > 0 ? 1 : 0; kk < (kDir > 0 ? 9 : 8); ++kk) {
+    const int zz = kDir > 0 ? z0 - 5 + kk : z1 - 4 + kk;
     float2 v = (v0 || v1)
                    ? __ldg(reinterpret_cast<const float2*>(bp.cz + (long long)zz * a.d.plane + off))
                    : make_float2(0.f, 0.f);
     // planes of the block above z0 were already damped as "cur"
-    if (!kExact && damp && zz >= 0 && (zz >> 2) < (z0 >> 2)) {
+    if (kDir > 0 && !kExact && damp && zz >= 0 && (zz >> 2) < (z0 >> 2)) {
       v.x *= dxy[0] * a.dampz[zz];
       v.y *= dxy[1] * a.dampz[zz];
     }
     q[kk] = v;
   }
-  // z damping factors in registers: dzr holds planes z-3..z once plane z
-  // is entered (the block transition rescales those four queue entries);
-  // the next plane's factor is fetched one plane ahead
-  float dzr[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) dzr[j] = (damp && z0 - 4 + j >= 0) ? a.dampz[z0 - 4 + j] : 1.f;
-  float dz_next = damp ? a.dampz[z0] : 1.f;
-  for (int z = z0; z < z1; ++z, k.advance()) {
-    const float dz = dz_next;
-    if (damp && z + 1 < z1) dz_next = a.dampz[z + 1];
-#pragma unroll
-    for (int j = 0; j < 3; ++j) dzr[j] = dzr[j + 1];
-    dzr[3] = dz;
+  int z = kDir > 0 ? z0 : z1 - 1;
+  const int zend = kDir > 0 ? z1 : z0 - 1;
+  long long i = (long long)z * a.d.plane + off;
+  const long long istep = kDir > 0 ? a.d.plane : -a.d.plane;
+  for (; z != zend; z += kDir, i += istep, k.advance()) {
+    const float dz = damp ? __ldg(a.dampz + z) : 1.f;
     // the model pair: loads issued before the stage wait
     float2 c11, c13, c33;
-    model_pair(a.c11, a.c13, a.c33, (long long)z * a.d.plane + off, v0 || v1, c11, c13, c33);
+    model_pair(a.c11, a.c13, a.c33, i, v0 || v1, c11, c13, c33);
     const int s = k.s;
     if (!mbar_wait(&full[s], k.ph, status)) return false;
     const unsigned char* st = smem + s * F_STAGE_BYTES;
     const float* sh = (const float*)(st + F_OFF_H) + sr;
     const float* pl = (const float*)(st + F_OFF_Z) + pi;  // [z+4][prev x][prev z]
     constexpr int T = TX * TY;
-#pragma unroll
-    for (int kk = 0; kk < 8; ++kk) q[kk] = q[kk + 1];
-    q[8] = ld2(pl);
+    queue_shift<kDir>(q, ld2(pl));
     // the row x-4 .. x+5 and the column pairs y +- 1..4
     float r[10];
 #pragma unroll
@@ -247,14 +304,18 @@ __device__ __forceinline__ bool fwd_consume(const FwdCommon& a, const FwdPar& bp
       lxx.x = lap9(r[4], r[3], r[5], r[2], r[6], r[1], r[7], r[0], r[8]);
       lxx.y = lap9(r[5], r[4], r[6], r[3], r[7], r[2], r[8], r[1], r[9]);
       const float2 lyy = lap9_2(c2, ym[0], yp[0], ym[1], yp[1], ym[2], yp[2], ym[3], yp[3]);
-      const float2 lzz = lap9_2(q[4], q[3], q[5], q[2], q[6], q[1], q[7], q[0], q[8]);
+      float2 u[4] = {q[0], q[1], q[2], q[3]};  // the planes above, as the stencil reads them
+      if (kDir < 0 && damp) damp_above(u, dxy, a.dampz, z);
+      const float2 lzz = lap9_2(q[4], u[3], q[5], u[2], q[6], u[1], q[7], u[0], q[8]);
       const float2 lxy = fma2(lyy, splat(a.sy), mul2(lxx, splat(a.sx)));
       const float2 lz = mul2(lzz, splat(a.sz));
       const float2 dd = mul2(make_float2(dxy[0], dxy[1]), splat(dz));
       const float2 ndd = mul2(dd, splat(-1.f));
       // 2 cur - dd prev, rounded once
-      float2 nx = fma2(c11, lxy, fma2(c13, lz, fma2(ndd, px, mul2(splat(2.f), c2))));
-      float2 nz = fma2(c13, lxy, fma2(c33, lz, fma2(ndd, pz, mul2(splat(2.f), q[4]))));
+      const bool on = kSponge != kSpongeOff;
+      const float2 wx = mul2(splat(2.f), c2), wz = mul2(splat(2.f), q[4]);
+      float2 nx = fma2(c11, lxy, fma2(c13, lz, on ? fma2(ndd, px, wx) : sub2(wx, px)));
+      float2 nz = fma2(c13, lxy, fma2(c33, lz, on ? fma2(ndd, pz, wz) : sub2(wz, pz)));
       if (kProbe && z == probe.z) {
         if (prb_e == 0) *probe.out += nx.x + nz.x;
         if (prb_e == 1) *probe.out += nx.y + nz.y;
@@ -269,14 +330,15 @@ __device__ __forceinline__ bool fwd_consume(const FwdCommon& a, const FwdPar& bp
           nz.y += amp;
         }
       }
-      nx = mul2(nx, dd);
-      nz = mul2(nz, dd);
+      if (on) {
+        nx = mul2(nx, dd);
+        nz = mul2(nz, dd);
+      }
       nxv[0] = nx.x;
       nxv[1] = nx.y;
       nzv[0] = nz.x;
       nzv[1] = nz.y;
     }
-    const long long i = (long long)z * a.d.plane + off;
     if (v0 && v1) {
       *reinterpret_cast<float2*>(bp.px + i) = make_float2(nxv[0], nxv[1]);
       *reinterpret_cast<float2*>(bp.pz + i) = make_float2(nzv[0], nzv[1]);
@@ -290,38 +352,34 @@ __device__ __forceinline__ bool fwd_consume(const FwdCommon& a, const FwdPar& bp
         bp.pz[i + 1] = nzv[1];
       }
     }
-    // entering the next plane: if it starts a new 4-plane block of the same
-    // column, the four planes of the block just finished become "damped cur"
-    if (!kExact && damp && ((z + 1) & 3) == 0 && z + 1 < a.d.nz) {
-      // after the shift at z+1, entries 0..3 hold planes z-3..z; they are
-      // entries 1..4 now
-#pragma unroll
-      for (int kk = 0; kk < 4; ++kk)
-        q[kk + 1] = mul2(q[kk + 1], make_float2(dxy[0] * dzr[kk], dxy[1] * dzr[kk]));
-    }
+    if (kDir > 0 && !kExact && damp) damp_finished_block(q, dxy, a.dampz, z, a.d.nz);
   }
   return true;
 }
 
 // kProbe: the probe point of FwdArgs is read out (wavelet gradient); the
 // propagation kernels are instantiated without it.
-template <bool kProbe, bool kExact>
+template <bool kProbe, bool kExact, int kDir, int kSponge>
 __global__ void __launch_bounds__(NTHREADS, 3)
     k_fwd3d_tma(const __grid_constant__ FwdMaps m0, const __grid_constant__ FwdArgs a0) {
   extern __shared__ unsigned char smem_raw[];
   uint64_t *full, *empty;
   unsigned char* smem = ring_init<F_STAGES, F_STAGE_BYTES>(smem_raw, full, empty);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  RingPos<F_STAGES> k;  // planes issued / consumed by this CTA
+  RingPos<F_STAGES> k;
   if (warp == NCW) {  // ---------------- producer
     if (lane == 0)
       for (int it = blockIdx.x; it < a0.c.sc.items; it += gridDim.x)
-        if (!fwd_produce(a0.c, m0, a0.status, it, smem, full, empty, k)) break;
+        if (!fwd_produce<kDir>(a0.c, m0, a0.status, march_item<kDir>(it, a0.c.sc.items), smem, full,
+                               empty, k))
+          break;
     return;
   }
   for (int it = blockIdx.x; it < a0.c.sc.items; it += gridDim.x)
-    if (!fwd_consume<kProbe, kExact>(a0.c, a0.p, a0.probe, a0.status, it, a0.c.src.amp, smem,
-                                     full, empty, k, warp, lane))
+    if (!fwd_consume<kProbe, kExact, kDir, kSponge>(a0.c, a0.p, a0.probe, a0.status,
+                                                    march_item<kDir>(it, a0.c.sc.items),
+                                                    a0.c.src.amp, smem, full, empty, k, warp,
+                                                    lane))
       break;
 }
 
@@ -354,6 +412,7 @@ __device__ __forceinline__ int find_job(const Batch& b, int item) {
   return lo;
 }
 
+template <int kDir>
 __global__ void __launch_bounds__(NTHREADS, 3) k_fwd3d_batch(const __grid_constant__ FwdBatch B) {
   extern __shared__ unsigned char smem_raw[];
   uint64_t *full, *empty;
@@ -362,20 +421,22 @@ __global__ void __launch_bounds__(NTHREADS, 3) k_fwd3d_batch(const __grid_consta
   RingPos<F_STAGES> k;
   if (warp == NCW) {
     if (lane == 0)
-      for (int it = blockIdx.x; it < B.items; it += gridDim.x) {
+      for (int n = blockIdx.x; n < B.items; n += gridDim.x) {
+        const int it = march_item<kDir>(n, B.items);
         const int j = find_job(B, it);
         const int par = (B.tick - B.c[j].t0) & 1;
-        if (!fwd_produce(B.c[j], B.maps[2 * j + par], B.status, it - B.base[j], smem, full,
+        if (!fwd_produce<kDir>(B.c[j], B.maps[2 * j + par], B.status, it - B.base[j], smem, full,
                          empty, k))
           break;
       }
     return;
   }
   const Probe none;
-  for (int it = blockIdx.x; it < B.items; it += gridDim.x) {
+  for (int n = blockIdx.x; n < B.items; n += gridDim.x) {
+    const int it = march_item<kDir>(n, B.items);
     const int j = find_job(B, it);
     const int step = B.tick - B.c[j].t0;
-    if (!fwd_consume<false>(B.c[j], B.p[j][step & 1], none, B.status, it - B.base[j],
+    if (!fwd_consume<false, false, kDir, kSpongeByJob>(B.c[j], B.p[j][step & 1], none, B.status, it - B.base[j],
                             __ldg(B.c[j].amp + step), smem, full, empty, k, warp, lane))
       break;
   }
@@ -435,14 +496,16 @@ struct BwdMaps {
 // wave3d.h:5-6 recording / imaging weights, as float
 constexpr float kTwoThirdF = (float)kTwoThird, kOneThirdF = (float)kOneThird;
 
-template <bool kRtm>
+template <bool kRtm, int kDir>
 __device__ __forceinline__ bool bwd_produce(const BwdCommon& a, const BwdMaps& m, int* status,
                                             int li, unsigned char* smem, uint64_t* full,
                                             uint64_t* empty, RingPos<B_STAGES>& k) {
   int bx, by, z0, z1;
   item(a.sc, li, bx, by, z0, z1);
   const int x0 = bx * TX, y0 = kHalo + by * TY;
-  for (int z = z0; z < z1; ++z, k.advance()) {
+  const int nz = z1 - z0;
+  for (int n = 0; n < nz; ++n, k.advance()) {
+    const int z = kDir > 0 ? z0 + n : z1 - 1 - n;
     const int s = k.s;
     if (!mbar_wait(&empty[s], k.ph ^ 1u, status)) return false;
     const int zp = z + kZPad;
@@ -451,8 +514,8 @@ __device__ __forceinline__ bool bwd_produce(const BwdCommon& a, const BwdMaps& m
     mbar_arrive_expect_tx(&full[s], B_STAGE_BYTES);
     tma_load(st + B_OFF_SH, &m.scx, &full[s], x0 - kHalo, y0 - kHalo, zp);
     tma_load(st + B_OFF_LH, &m.lcx, &full[s], x0 - kHalo, y0 - kHalo, zp);
-    tma_load(pl + 0 * PLAIN_BYTES, &m.scz, &full[s], x0, y0, zp + kHalo);
-    tma_load(pl + 1 * PLAIN_BYTES, &m.lcz, &full[s], x0, y0, zp + kHalo);
+    tma_load(pl + 0 * PLAIN_BYTES, &m.scz, &full[s], x0, y0, zp + kDir * kHalo);
+    tma_load(pl + 1 * PLAIN_BYTES, &m.lcz, &full[s], x0, y0, zp + kDir * kHalo);
     tma_load(pl + 2 * PLAIN_BYTES, &m.spx, &full[s], x0, y0, zp);
     tma_load(pl + 3 * PLAIN_BYTES, &m.spz, &full[s], x0, y0, zp);
     tma_load(pl + 4 * PLAIN_BYTES, &m.lpx, &full[s], x0, y0, zp);
@@ -462,7 +525,7 @@ __device__ __forceinline__ bool bwd_produce(const BwdCommon& a, const BwdMaps& m
 }
 
 // Consumers: the x pair x0 + 2*(lane%16) + {0,1} of tile row 2*warp + lane/16.
-template <bool kRtm>
+template <bool kRtm, int kDir>
 __device__ __forceinline__ bool bwd_consume(const BwdCommon& a, const BwdPar& bp, int* status,
                                             int li, float amp, const unsigned char* smem,
                                             uint64_t* full, uint64_t* empty, RingPos<B_STAGES>& k,
@@ -483,48 +546,42 @@ __device__ __forceinline__ bool bwd_consume(const BwdCommon& a, const BwdPar& bp
   const int off = y * a.d.pitch + x;  // x + 1 < pitch: 32 * gx <= pitch
   dxy[0] = v0 ? a.dampx[x] * a.dampy[y] : 1.f;
   dxy[1] = v1 ? a.dampx[x + 1] * a.dampy[y] : 1.f;
-  // start the queues: planes z0-4 .. z0+3 from global
-  sq[0] = lq[0] = make_float2(0.f, 0.f);
+  // start the queues from global (planes as in the forward kernel)
+  sq[kDir > 0 ? 0 : 8] = lq[kDir > 0 ? 0 : 8] = make_float2(0.f, 0.f);
 #pragma unroll
-  for (int kk = 1; kk < 9; ++kk) {
-    const int zz = z0 - 5 + kk;
+  for (int kk = kDir > 0 ? 1 : 0; kk < (kDir > 0 ? 9 : 8); ++kk) {
+    const int zz = kDir > 0 ? z0 - 5 + kk : z1 - 4 + kk;
     const long long i = (long long)zz * a.d.plane + off;
     const bool any = v0 || v1;
     const float2 sv =
         any ? __ldg(reinterpret_cast<const float2*>(bp.scz + i)) : make_float2(0.f, 0.f);
     float2 lv = any ? __ldg(reinterpret_cast<const float2*>(bp.lcz + i)) : make_float2(0.f, 0.f);
-    if (zz >= 0 && (zz >> 2) < (z0 >> 2)) {
+    if (kDir > 0 && zz >= 0 && (zz >> 2) < (z0 >> 2)) {
       lv.x *= dxy[0] * a.dampz[zz];
       lv.y *= dxy[1] * a.dampz[zz];
     }
     sq[kk] = sv;
     lq[kk] = lv;
   }
-  // z damping factors in registers (see the forward kernel)
-  float dzr[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) dzr[j] = z0 - 4 + j >= 0 ? a.dampz[z0 - 4 + j] : 1.f;
-  float dz_next = a.dampz[z0];
   // this thread's gradient pair of a plane (read with plain loads)
   const bool anyv = v0 || v1;
-  auto gload = [&](int zz, float2& r11, float2& r13, float2& r33) {
-    const long long i = (long long)zz * a.d.plane + off;
+  auto gload = [&](long long i, float2& r11, float2& r13, float2& r33) {
     const float2 zero = make_float2(0.f, 0.f);
     r11 = anyv ? __ldg(reinterpret_cast<const float2*>(a.g11 + i)) : zero;
     r13 = (anyv && !kRtm) ? __ldg(reinterpret_cast<const float2*>(a.g13 + i)) : zero;
     r33 = (anyv && !kRtm) ? __ldg(reinterpret_cast<const float2*>(a.g33 + i)) : zero;
   };
-  for (int z = z0; z < z1; ++z, k.advance()) {
-    const float dz = dz_next;
-    if (z + 1 < z1) dz_next = a.dampz[z + 1];
+  int z = kDir > 0 ? z0 : z1 - 1;
+  const int zend = kDir > 0 ? z1 : z0 - 1;
+  long long i = (long long)z * a.d.plane + off;
+  const long long istep = kDir > 0 ? a.d.plane : -a.d.plane;
+  for (; z != zend; z += kDir, i += istep, k.advance()) {
+    const float dz = __ldg(a.dampz + z);
     // issued before the stage wait: the loads complete while the stage
     // arrives and the stencils are evaluated
     float2 g11o, g13o, g33o, c11, c13, c33;
-    gload(z, g11o, g13o, g33o);
-    model_pair(a.c11, a.c13, a.c33, (long long)z * a.d.plane + off, anyv, c11, c13, c33);
-#pragma unroll
-    for (int j = 0; j < 3; ++j) dzr[j] = dzr[j + 1];
-    dzr[3] = dz;
+    gload(i, g11o, g13o, g33o);
+    model_pair(a.c11, a.c13, a.c33, i, anyv, c11, c13, c33);
     const int s = k.s;
     if (!mbar_wait(&full[s], k.ph, status)) return false;
     const unsigned char* st = smem + s * B_STAGE_BYTES;
@@ -532,13 +589,8 @@ __device__ __forceinline__ bool bwd_consume(const BwdCommon& a, const BwdPar& bp
     const float* lh = (const float*)(st + B_OFF_LH) + sr;
     const float* pl = (const float*)(st + B_OFF_P) + pi;
     constexpr int T = TX * TY;
-#pragma unroll
-    for (int kk = 0; kk < 8; ++kk) {
-      sq[kk] = sq[kk + 1];
-      lq[kk] = lq[kk + 1];
-    }
-    sq[8] = ld2(pl);
-    lq[8] = ld2(pl + T);
+    queue_shift<kDir>(sq, ld2(pl));
+    queue_shift<kDir>(lq, ld2(pl + T));
     // x rows (x-4 .. x+5) and y column pairs of both halo fields
     float rs[10], rl[10];
 #pragma unroll
@@ -576,10 +628,11 @@ __device__ __forceinline__ bool bwd_consume(const BwdCommon& a, const BwdPar& bp
     lxx.x = lap9(rl[4], rl[3], rl[5], rl[2], rl[6], rl[1], rl[7], rl[0], rl[8]);
     lxx.y = lap9(rl[5], rl[4], rl[6], rl[3], rl[7], rl[2], rl[8], rl[1], rl[9]);
     const float2 szz = lap9_2(sq[4], sq[3], sq[5], sq[2], sq[6], sq[1], sq[7], sq[0], sq[8]);
-    const float2 lzz = lap9_2(lq[4], lq[3], lq[5], lq[2], lq[6], lq[1], lq[7], lq[0], lq[8]);
+    float2 u[4] = {lq[0], lq[1], lq[2], lq[3]};
+    if (kDir < 0) damp_above(u, dxy, a.dampz, z);
+    const float2 lzz = lap9_2(lq[4], u[3], lq[5], u[2], lq[6], u[1], lq[7], u[0], lq[8]);
     const float2 sxy_u = fma2(syy, splat(a.idy2), mul2(sxx, splat(a.idx2)));
     const float2 sz_u = mul2(szz, splat(a.idz2));
-    const long long i = (long long)z * a.d.plane + off;
     // each result pair is stored as soon as it is complete (shorter live
     // ranges: the whole step fits the 96 registers of two CTAs per SM)
     auto store2 = [&](float* f, float2 v) {
@@ -624,11 +677,7 @@ __device__ __forceinline__ bool bwd_consume(const BwdCommon& a, const BwdPar& bp
     // 2 cur - dd prev, rounded once
     store2(bp.lpx, mul2(dd, fma2(c11, lxy, fma2(c13, lzs, fma2(ndd, lpx, mul2(two, lc))))));
     store2(bp.lpz, mul2(dd, fma2(c13, lxy, fma2(c33, lzs, fma2(ndd, lpz, mul2(two, lz0))))));
-    if (((z + 1) & 3) == 0 && z + 1 < a.d.nz) {
-#pragma unroll
-      for (int kk = 0; kk < 4; ++kk)
-        lq[kk + 1] = mul2(lq[kk + 1], make_float2(dxy[0] * dzr[kk], dxy[1] * dzr[kk]));
-    }
+    if (kDir > 0) damp_finished_block(lq, dxy, a.dampz, z, a.d.nz);
   }
   return true;
 }
@@ -638,7 +687,7 @@ __device__ __forceinline__ bool bwd_consume(const BwdCommon& a, const BwdPar& bp
 // (2/3 sx + 1/3 sz)(2/3 lx + 1/3 lz) with both fields at the current level and
 // the adjoint already multiplied by this step's sponge; g13/g33 are neither
 // loaded nor written.
-template <bool kRtm>
+template <bool kRtm, int kDir>
 __global__ void __launch_bounds__(NTHREADS, 2)
     k_bwd3d_tma(const __grid_constant__ BwdMaps m0, const __grid_constant__ BwdArgs a0) {
   extern __shared__ unsigned char smem_raw[];
@@ -649,12 +698,14 @@ __global__ void __launch_bounds__(NTHREADS, 2)
   if (warp == NCW) {
     if (lane == 0)
       for (int it = blockIdx.x; it < a0.c.sc.items; it += gridDim.x)
-        if (!bwd_produce<kRtm>(a0.c, m0, a0.status, it, smem, full, empty, k)) break;
+        if (!bwd_produce<kRtm, kDir>(a0.c, m0, a0.status, march_item<kDir>(it, a0.c.sc.items), smem,
+                                     full, empty, k))
+          break;
     return;
   }
   for (int it = blockIdx.x; it < a0.c.sc.items; it += gridDim.x)
-    if (!bwd_consume<kRtm>(a0.c, a0.p, a0.status, it, a0.c.src.amp, smem, full, empty, k, warp,
-                           lane))
+    if (!bwd_consume<kRtm, kDir>(a0.c, a0.p, a0.status, march_item<kDir>(it, a0.c.sc.items),
+                                 a0.c.src.amp, smem, full, empty, k, warp, lane))
       break;
 }
 
@@ -667,6 +718,7 @@ struct BwdBatch {
   BwdPar p[kMaxBwdJobs][2];
 };
 
+template <int kDir>
 __global__ void __launch_bounds__(NTHREADS, 2) k_bwd3d_batch(const __grid_constant__ BwdBatch B) {
   extern __shared__ unsigned char smem_raw[];
   uint64_t *full, *empty;
@@ -675,19 +727,21 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_bwd3d_batch(const __grid_consta
   RingPos<B_STAGES> k;
   if (warp == NCW) {
     if (lane == 0)
-      for (int it = blockIdx.x; it < B.items; it += gridDim.x) {
+      for (int n = blockIdx.x; n < B.items; n += gridDim.x) {
+        const int it = march_item<kDir>(n, B.items);
         const int j = find_job(B, it);
         const int par = (B.tick - B.c[j].t0) & 1;
-        if (!bwd_produce<false>(B.c[j], B.maps[2 * j + par], B.status, it - B.base[j], smem,
+        if (!bwd_produce<false, kDir>(B.c[j], B.maps[2 * j + par], B.status, it - B.base[j], smem,
                                 full, empty, k))
           break;
       }
     return;
   }
-  for (int it = blockIdx.x; it < B.items; it += gridDim.x) {
+  for (int n = blockIdx.x; n < B.items; n += gridDim.x) {
+    const int it = march_item<kDir>(n, B.items);
     const int j = find_job(B, it);
     const int step = B.tick - B.c[j].t0;
-    if (!bwd_consume<false>(B.c[j], B.p[j][step & 1], B.status, it - B.base[j],
+    if (!bwd_consume<false, kDir>(B.c[j], B.p[j][step & 1], B.status, it - B.base[j],
                             __ldg(B.c[j].amp + step), smem, full, empty, k, warp, lane))
       break;
   }
@@ -844,7 +898,7 @@ FwdCommon fwd_common(const Dims3& d, const Sched& sc, const Damping* damp, float
   return c;
 }
 
-std::atomic<bool> attr_fwd[3][64], attr_bwd[2][64], attr_fwd_batch[64], attr_bwd_batch[64];
+std::atomic<bool> attr_fwd[8][64], attr_bwd[4][64], attr_fwd_batch[2][64], attr_bwd_batch[2][64];
 
 }  // namespace
 
@@ -852,12 +906,19 @@ int launch_fwd3d_tma(vti_ctx* ctx, const Dims3& d, const TileMaps& cx, const Til
                      const TileMaps& px, const TileMaps& pz, const TileMaps& c11,
                      const TileMaps& c13, const TileMaps& c33, const float* cz_ptr,
                      float* px_ptr, float* pz_ptr, const Damping* damp, float sx, float sy,
-                     float sz, PointSource src, Probe probe, bool exact) {
+                     float sz, PointSource src, Probe probe, bool exact, bool up) {
   const bool pr = probe.x >= 0 && probe.out;
   if (pr && exact) return fail(ctx, VTI_ERR_UNSUPPORTED, "probe with the exact-mode step");
-  auto kern = pr ? k_fwd3d_tma<true, false>
-                 : (exact ? k_fwd3d_tma<false, true> : k_fwd3d_tma<false, false>);
-  const int variant = pr ? 1 : (exact ? 2 : 0);
+  constexpr int kOff = kSpongeOff, kOn = kSpongeOn;
+  void (*const kerns[8])(FwdMaps, FwdArgs) = {
+      k_fwd3d_tma<false, false, 1, kOff>, k_fwd3d_tma<false, false, -1, kOff>,
+      k_fwd3d_tma<false, false, 1, kOn>,  k_fwd3d_tma<false, false, -1, kOn>,
+      k_fwd3d_tma<true, false, 1, kOn>,   k_fwd3d_tma<true, false, -1, kOn>,
+      k_fwd3d_tma<false, true, 1, kOn>,   k_fwd3d_tma<false, true, -1, kOn>};
+  if ((pr || exact) && !damp)
+    return fail(ctx, VTI_ERR_UNSUPPORTED, "probe / exact-mode step without the sponge");
+  const int variant = 2 * (pr ? 2 : (exact ? 3 : (damp ? 1 : 0))) + (up ? 1 : 0);
+  const auto kern = kerns[variant];
   VTI_TRY_ST(set_smem_attr(ctx, kern, F_SMEM, attr_fwd[variant]));
   FwdMaps m;
   m.cx = *H(cx); m.cz = *P(cz); m.px = *P(px); m.pz = *P(pz);
@@ -883,9 +944,12 @@ int launch_bwd3d_tma(vti_ctx* ctx, const Dims3& d, const TileMaps& scx, const Ti
                      const float* scz_ptr, const float* lcz_ptr, float* spx_ptr, float* spz_ptr,
                      float* lpx_ptr, float* lpz_ptr, float* g11_ptr, float* g13_ptr,
                      float* g33_ptr, const Damping& damp, float dt2, float idx2, float idy2,
-                     float idz2, float sx, float sy, float sz, PointSource src, bool rtm) {
-  VTI_TRY_ST(set_smem_attr(ctx, rtm ? k_bwd3d_tma<true> : k_bwd3d_tma<false>, B_SMEM,
-                           attr_bwd[rtm]));
+                     float idz2, float sx, float sy, float sz, PointSource src, bool rtm, bool up) {
+  void (*const kerns[4])(BwdMaps, BwdArgs) = {k_bwd3d_tma<false, 1>, k_bwd3d_tma<false, -1>,
+                                              k_bwd3d_tma<true, 1>, k_bwd3d_tma<true, -1>};
+  const int variant = 2 * (rtm ? 1 : 0) + (up ? 1 : 0);
+  const auto kern = kerns[variant];
+  VTI_TRY_ST(set_smem_attr(ctx, kern, B_SMEM, attr_bwd[variant]));
   BwdMaps m;
   m.scx = *H(scx); m.scz = *P(scz); m.spx = *P(spx); m.spz = *P(spz);
   m.lcx = *H(lcx); m.lcz = *P(lcz); m.lpx = *P(lpx); m.lpz = *P(lpz);
@@ -904,10 +968,7 @@ int launch_bwd3d_tma(vti_ctx* ctx, const Dims3& d, const TileMaps& scx, const Ti
   const int grid = c.sc.grid;
   {
     LaunchTimer tm(ctx, kTimedBwd3d);
-    if (rtm)
-      k_bwd3d_tma<true><<<grid, NTHREADS, B_SMEM, ctx->stream>>>(m, a);
-    else
-      k_bwd3d_tma<false><<<grid, NTHREADS, B_SMEM, ctx->stream>>>(m, a);
+    kern<<<grid, NTHREADS, B_SMEM, ctx->stream>>>(m, a);
   }
   VTI_LAUNCHED(ctx, "k_bwd3d_tma");
   return VTI_OK;
@@ -924,8 +985,10 @@ struct StepBatch {
 };
 
 int prepare_batch_kernels(vti_ctx* ctx) {
-  VTI_TRY_ST(set_smem_attr(ctx, k_fwd3d_batch, F_SMEM, attr_fwd_batch));
-  VTI_TRY_ST(set_smem_attr(ctx, k_bwd3d_batch, B_SMEM, attr_bwd_batch));
+  VTI_TRY_ST(set_smem_attr(ctx, k_fwd3d_batch<1>, F_SMEM, attr_fwd_batch[0]));
+  VTI_TRY_ST(set_smem_attr(ctx, k_fwd3d_batch<-1>, F_SMEM, attr_fwd_batch[1]));
+  VTI_TRY_ST(set_smem_attr(ctx, k_bwd3d_batch<1>, B_SMEM, attr_bwd_batch[0]));
+  VTI_TRY_ST(set_smem_attr(ctx, k_bwd3d_batch<-1>, B_SMEM, attr_bwd_batch[1]));
   return VTI_OK;
 }
 
@@ -1052,7 +1115,8 @@ int step_batch_launch(vti_ctx* ctx, StepBatch* b, int tick) {
       const int grid = std::min(B.items, ctx->sm_count * 3);
       {
         LaunchTimer tm(ctx, kTimedFwd3d);
-        k_fwd3d_batch<<<grid, NTHREADS, F_SMEM, ctx->stream>>>(B);
+        const auto kern = tick & 1 ? k_fwd3d_batch<-1> : k_fwd3d_batch<1>;
+        kern<<<grid, NTHREADS, F_SMEM, ctx->stream>>>(B);
       }
       VTI_LAUNCHED(ctx, "k_fwd3d_batch");
     }
@@ -1063,7 +1127,8 @@ int step_batch_launch(vti_ctx* ctx, StepBatch* b, int tick) {
       const int grid = std::min(B.items, ctx->sm_count * 2);
       {
         LaunchTimer tm(ctx, kTimedBwd3d);
-        k_bwd3d_batch<<<grid, NTHREADS, B_SMEM, ctx->stream>>>(B);
+        const auto kern = tick & 1 ? k_bwd3d_batch<-1> : k_bwd3d_batch<1>;
+        kern<<<grid, NTHREADS, B_SMEM, ctx->stream>>>(B);
       }
       VTI_LAUNCHED(ctx, "k_bwd3d_batch");
     }
