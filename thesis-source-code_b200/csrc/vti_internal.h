@@ -89,25 +89,42 @@ struct NvtxRange {
   NvtxRange(const NvtxRange&) = delete;
   NvtxRange& operator=(const NvtxRange&) = delete;
 };
-// Launch with programmatic stream serialization: the kernel may start while
-// the previous kernel of the stream runs; it must execute griddepcontrol.wait
-// before it touches anything the previous kernels write (launched normally,
-// the wait returns at once).
+// Launch with (early) or without programmatic stream serialization. With it
+// the kernel may start while the previous kernel of the stream runs; it must
+// execute griddepcontrol.wait before it touches anything the previous kernels
+// write (launched normally, the wait returns at once).
 template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream_t s,
-                       Args&&... args) {
+cudaError_t launch_ex(bool early, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                      cudaStream_t s, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = early ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream_t s,
+                       Args&&... args) {
+  return launch_ex(true, kern, grid, block, 0, s, std::forward<Args>(args)...);
+}
+#ifdef __CUDACC__
+// First statement of a kernel launched early: lets the next launch of the
+// stream become resident as this one's CTAs finish.
+__device__ __forceinline__ void pdl_launch_next() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// Returns when the launches before this one have finished and their writes
+// are visible; every thread calls it before it touches anything they write.
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+#endif
 // Brackets one launch with events on ctx->stream when timing is enabled.
 struct LaunchTimer {
   vti_ctx* ctx;
@@ -280,11 +297,20 @@ int wait_selftest(vti_ctx* ctx, unsigned polls);
 int check_device_status(vti_ctx* ctx);
 
 // Sparse receiver kernels. rec: device offsets (Dims3::off) per receiver.
+// early: launch_ex's, see receivers_early.
 int launch_record(vti_ctx* ctx, float* trace, int nnt, int j, const float* cx, const float* cz,
-                  const long long* rec, int nr);
+                  const long long* rec, int nr, bool early = false);
 int launch_inject_residual(vti_ctx* ctx, float* lx, float* lz, const float* res, int nnt,
                            int i0, float f, int clamp_last, const long long* rec,
-                           const float* rec_damp, int nr, float dt2);
+                           const float* rec_damp, int nr, float dt2, bool early = false);
+// Whether the receiver launch after a step that moves bytes_per_point of every
+// point of d is an early one: it saves the launch gap (gradient 80x80x64, 299
+// levels: 10.3 -> 9.5 ms, 176x176x128 37.7 -> 36.9 ms), but from about 300 MB per
+// step on its CTAs, resident beside the step's last ones, cost more than that
+// (208x192x128 46.3 -> 47.5 ms).
+inline bool receivers_early(const Dims3& d, int bytes_per_point) {
+  return d.npoints() * bytes_per_point <= 320000000LL;
+}
 int launch_seed_adjoint(vti_ctx* ctx, float* lx, float* lz, const float* res, int nnt,
                         const long long* rec, const float* rec_damp, int nr, float dt2);
 int launch_set_point(vti_ctx* ctx, float* a, float* b, long long off, float value);

@@ -30,6 +30,8 @@ namespace {
 // recordData (injectRecord3d.cu:22-28) into trace-major traces.
 __global__ void k_record(float* trace, int nnt, int j, const float* cx, const float* cz,
                          const long long* rec, int nr) {
+  pdl_launch_next();
+  pdl_wait();
   int ir = blockIdx.x * blockDim.x + threadIdx.x;
   if (ir < nr) {
     long long o = rec[ir];
@@ -43,6 +45,8 @@ __global__ void k_record(float* trace, int nnt, int j, const float* cx, const fl
 __global__ void k_inject_residual(float* lx, float* lz, const float* res, int nnt, int i0,
                                   float f, int clamp_last, const long long* rec,
                                   const float* rec_damp, int nr, float dt2) {
+  pdl_launch_next();
+  pdl_wait();
   int ir = blockIdx.x * blockDim.x + threadIdx.x;
   if (ir < nr) {
     const float* t = res + (long long)ir * nnt;
@@ -276,19 +280,20 @@ int launch_odcig3d(vti_ctx* ctx, const Dims3& d, const float* sx, const float* s
 }
 
 int launch_record(vti_ctx* ctx, float* trace, int nnt, int j, const float* cx, const float* cz,
-                  const long long* rec, int nr) {
+                  const long long* rec, int nr, bool early) {
   if (nr <= 0) return VTI_OK;
-  k_record<<<(nr + 255) / 256, 256, 0, ctx->stream>>>(trace, nnt, j, cx, cz, rec, nr);
+  VTI_CUDA(ctx, launch_ex(early, k_record, dim3((nr + 255) / 256), dim3(256), 0, ctx->stream, trace, nnt, j,
+                           cx, cz, rec, nr));
   VTI_LAUNCHED(ctx, "k_record");
   return VTI_OK;
 }
 
 int launch_inject_residual(vti_ctx* ctx, float* lx, float* lz, const float* res, int nnt,
                            int i0, float f, int clamp_last, const long long* rec,
-                           const float* rec_damp, int nr, float dt2) {
+                           const float* rec_damp, int nr, float dt2, bool early) {
   if (nr <= 0) return VTI_OK;
-  k_inject_residual<<<(nr + 255) / 256, 256, 0, ctx->stream>>>(lx, lz, res, nnt, i0, f,
-                                                               clamp_last, rec, rec_damp, nr, dt2);
+  VTI_CUDA(ctx, launch_ex(early, k_inject_residual, dim3((nr + 255) / 256), dim3(256), 0, ctx->stream, lx,
+                           lz, res, nnt, i0, f, clamp_last, rec, rec_damp, nr, dt2));
   VTI_LAUNCHED(ctx, "k_inject_residual");
   return VTI_OK;
 }

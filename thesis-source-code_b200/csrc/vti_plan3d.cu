@@ -225,7 +225,7 @@ int fwd_level(vti3d_plan* p, const ShotGeom& s, bool sponge, int A, int B, int i
                            dt2 / (g.dz * g.dz), src, Probe(), false, (it & 1) != 0));
   if (sponge && it < (int)s.rec_at.size() && s.rec_at[it] >= 0)
     VTI_TRY(launch_record(ctx, p->d_trace, nnt_of(g), s.rec_at[it], p->sx[B].origin,
-                          p->sz[B].origin, p->d_rec, s.nr));
+                          p->sz[B].origin, p->d_rec, s.nr, receivers_early(p->d, 36)));
   return VTI_OK;
 }
 
@@ -294,7 +294,8 @@ int bwd_level(vti3d_plan* p, const ShotGeom& s, bool rtm, int SA, int SB, int LA
   int clamp = i0 >= nnt - 1;
   f = f - i0;
   return launch_inject_residual(ctx, p->lx[LB].origin, p->lz[LB].origin, p->d_trace, nnt,
-                                clamp ? 0 : i0, f, clamp, p->d_rec, p->d_rec_damp, s.nr, dt2);
+                                clamp ? 0 : i0, f, clamp, p->d_rec, p->d_rec_damp, s.nr, dt2,
+                                receivers_early(p->d, rtm ? 68 : 84));
 }
 
 // Time-reversed source wavefield + adjoint + imaging (pass 3,
@@ -859,7 +860,7 @@ int vti3d_plan_wavelet_gradient(vti3d_plan* p, const float* souloc, const int* s
       f = f - i0;
       VTI_TRY(launch_inject_residual(ctx, p->lx[LB].origin, p->lz[LB].origin, p->d_trace, nnt,
                                      clamp ? 0 : i0, f, clamp, p->d_rec, p->d_rec_damp, s.nr,
-                                     dt2));
+                                     dt2, receivers_early(d, 36)));
       std::swap(LA, LB);
     }
     VTI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

@@ -362,9 +362,11 @@ __device__ __forceinline__ bool fwd_consume(const FwdCommon& a, const FwdPar& bp
 template <bool kProbe, bool kExact, int kDir, int kSponge>
 __global__ void __launch_bounds__(NTHREADS, 3)
     k_fwd3d_tma(const __grid_constant__ FwdMaps m0, const __grid_constant__ FwdArgs a0) {
+  pdl_launch_next();
   extern __shared__ unsigned char smem_raw[];
   uint64_t *full, *empty;
   unsigned char* smem = ring_init<F_STAGES, F_STAGE_BYTES>(smem_raw, full, empty);
+  pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   RingPos<F_STAGES> k;
   if (warp == NCW) {  // ---------------- producer
@@ -690,9 +692,11 @@ __device__ __forceinline__ bool bwd_consume(const BwdCommon& a, const BwdPar& bp
 template <bool kRtm, int kDir>
 __global__ void __launch_bounds__(NTHREADS, 2)
     k_bwd3d_tma(const __grid_constant__ BwdMaps m0, const __grid_constant__ BwdArgs a0) {
+  pdl_launch_next();
   extern __shared__ unsigned char smem_raw[];
   uint64_t *full, *empty;
   unsigned char* smem = ring_init<B_STAGES, B_STAGE_BYTES>(smem_raw, full, empty);
+  pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   RingPos<B_STAGES> k;
   if (warp == NCW) {
@@ -902,6 +906,18 @@ std::atomic<bool> attr_fwd[8][64], attr_bwd[4][64], attr_fwd_batch[2][64], attr_
 
 }  // namespace
 
+// Whether a step is launched early (programmatic dependent launch). It saves
+// the launch gap, about 2 us per level (128^3 modeling 15.5 -> 13.6 ms over 999
+// levels), but its CTAs land on whichever SMs finish first, so a column moves
+// to another SM, and half of the time to the other die's L2, from one level to
+// the next: 2 % on 400x400x200 and 251x203x150 gradients, whose launches last
+// 50 us and more. Hence only launches that move at most 250 MB (about 40 us).
+// With few CTAs (80x80x64: 120) early CTAs share SMs that others leave empty
+// (model 2.84 -> 3.24 ms over 299 levels): at least 1.5 per SM.
+static bool early_launch(vti_ctx* ctx, const Dims3& d, int bytes_per_point, int grid) {
+  return d.npoints() * bytes_per_point <= 250000000LL && 2 * grid >= 3 * ctx->sm_count;
+}
+
 int launch_fwd3d_tma(vti_ctx* ctx, const Dims3& d, const TileMaps& cx, const TileMaps& cz,
                      const TileMaps& px, const TileMaps& pz, const TileMaps& c11,
                      const TileMaps& c13, const TileMaps& c33, const float* cz_ptr,
@@ -930,7 +946,8 @@ int launch_fwd3d_tma(vti_ctx* ctx, const Dims3& d, const TileMaps& cx, const Til
   const int grid = a.c.sc.grid;
   {
     LaunchTimer tm(ctx, kTimedFwd3d);
-    kern<<<grid, NTHREADS, F_SMEM, ctx->stream>>>(m, a);
+    VTI_CUDA(ctx, launch_ex(early_launch(ctx, d, 36, grid), kern, dim3(grid), dim3(NTHREADS), F_SMEM,
+                            ctx->stream, m, a));
   }
   VTI_LAUNCHED(ctx, "k_fwd3d_tma");
   return VTI_OK;
@@ -968,7 +985,8 @@ int launch_bwd3d_tma(vti_ctx* ctx, const Dims3& d, const TileMaps& scx, const Ti
   const int grid = c.sc.grid;
   {
     LaunchTimer tm(ctx, kTimedBwd3d);
-    kern<<<grid, NTHREADS, B_SMEM, ctx->stream>>>(m, a);
+    VTI_CUDA(ctx, launch_ex(early_launch(ctx, d, rtm ? 68 : 84, grid), kern, dim3(grid), dim3(NTHREADS), B_SMEM,
+                            ctx->stream, m, a));
   }
   VTI_LAUNCHED(ctx, "k_bwd3d_tma");
   return VTI_OK;
