@@ -1,0 +1,42 @@
+"""Host arrays of pitched volumes (staged, packed and unpacked on the device) against device arrays of the same calls: equal bit for
+bit."""
+import numpy as np
+import pytest
+
+import vtib200 as V
+import vtib200.synth as S
+
+pytestmark = pytest.mark.gpu
+
+
+# below the staging limit; rows of one pitch; several planes; more than one
+# 32 MB block, with an output of more than 4 MB
+@pytest.mark.parametrize("nx,ny,nz", [(25, 21, 20), (64, 30, 24), (70, 41, 33), (250, 200, 190)])
+def test_host_and_device_arrays_agree(ctx, nx, ny, nz):
+    import torch
+    s = S.small3d(nx=nx, ny=ny, nz=nz, nt=12, npad=5, rate=2.1e-3)
+    n = s.nxyz
+    c = s.cij().reshape(3, n)
+    dobs = np.zeros(V.nnt3d(s.geom()) * (s.recloc.size // 4), dtype=np.float32)
+    res = []
+    for mem in (V.MEM_HOST, V.MEM_DEVICE):
+        plan = V.Plan3d(ctx, s.geom(), V.OPT_FULL_STEPS)
+        plan.set_wavelet(s.wavelet)
+        plan.set_receivers(s.recloc)
+        if mem == V.MEM_HOST:
+            plan.set_model(*c)
+            out = np.full(2 + 3 * n, np.nan, dtype=np.float32)[1:]  # not page aligned
+            plan.gradient(s.souloc, [0], dobs, V.MEM_HOST, out, V.MEM_HOST)
+            fresh = plan.gradient(s.souloc, [0], dobs)[0]
+            assert np.array_equal(out, fresh)
+        else:
+            dc = [torch.tensor(k, device="cuda") for k in c]
+            dd, fg = torch.tensor(dobs, device="cuda"), torch.zeros(1 + 3 * n, device="cuda")
+            torch.cuda.synchronize()
+            plan.set_model(*[k.data_ptr() for k in dc], mem=V.MEM_DEVICE)
+            plan.gradient(s.souloc, [0], dd.data_ptr(), V.MEM_DEVICE, fg.data_ptr(), V.MEM_DEVICE)
+            out = fg.cpu().numpy()
+        res.append(out)
+        plan.close()
+    assert np.abs(res[0][1:]).max() > 0
+    assert np.array_equal(res[0], res[1])

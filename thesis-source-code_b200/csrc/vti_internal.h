@@ -23,6 +23,9 @@ constexpr int kZPad = kHalo;
 // (wave3d.h:17) and therefore runs 2 + 64*floor((nt-2)/64) time levels.
 constexpr int kRefUpdate = 64;
 
+// Bytes of the staging block that host transfers of pitched volumes go through.
+constexpr size_t kStageBytes = (size_t)32 << 20;
+
 // Recording / injection weights (wave3d.h:5-6).
 constexpr double kTwoThird = 0.6666666666;
 constexpr double kOneThird = 0.3333333333;
@@ -72,6 +75,8 @@ struct vti_ctx {
   // device scratch of the 2D forward forms, kept between calls
   float* scratch2d = nullptr;
   size_t scratch2d_bytes = 0;
+  // staging block of host transfers of pitched volumes, kept between calls
+  float* stage = nullptr;
   // plan kept by the one-call 3D forms while their geometry and flags repeat
   bool plan_cache = true;
   vti3d_plan* cached_plan = nullptr;
@@ -162,6 +167,8 @@ int vol_zero(vti_ctx* ctx, const Dims3& d, Vol* v);
 // Contiguous x-fastest host/device array <-> pitched volume.
 int vol_upload(vti_ctx* ctx, const Dims3& d, Vol* v, const float* src, int mem);
 int vol_download(vti_ctx* ctx, const Dims3& d, const Vol* v, float* dst, int mem);
+// Pitched rows (plane 0 of a volume without z pad planes) -> contiguous array.
+int rows_download(vti_ctx* ctx, const Dims3& d, const float* rows, float* dst, int mem);
 
 Dims3 make_dims(int nx, int ny, int nz);
 

@@ -799,13 +799,9 @@ int vti3d_plan_odcig(vti3d_plan* p, const float* souloc, const int* shotid, int 
     VTI_TRY(backward_pass(p, s, true, p->d_ext, nlag));
     VTI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   }
-  const cudaMemcpyKind kind =
-      image_mem == VTI_MEM_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
   const size_t nxyz = (size_t)d.nx * d.ny * d.nz;
   for (int l = 0; l < nl; ++l)
-    VTI_CUDA(ctx, cudaMemcpy2DAsync(image + l * nxyz, d.nx * sizeof(float), p->d_ext + l * vol,
-                                    d.pitch * sizeof(float), d.nx * sizeof(float),
-                                    (size_t)d.ny * d.nz, kind, ctx->stream));
+    VTI_TRY(rows_download(ctx, d, p->d_ext + l * vol, image + l * nxyz, image_mem));
   VTI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return check_device_status(ctx);
 }

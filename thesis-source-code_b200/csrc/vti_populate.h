@@ -1,0 +1,76 @@
+// Destination pages of a host download, populated by helper threads while the
+// device computes.
+//
+// A caller's fresh array (calloc, np.zeros) has no pages yet: the copy that
+// first writes it takes a page fault per 4 KB in the one thread that feeds the
+// copy, 2.3 GB/s instead of 17 for a 115 MB download. MADV_POPULATE_WRITE makes
+// the pages writable without changing what they hold, so it is safe on arrays
+// in any state, and a kernel without it returns an error that is ignored.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
+
+#include <algorithm>
+#include <cstdint>
+#include <system_error>
+#include <thread>
+#include <vector>
+
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+
+namespace vti {
+
+class Populate {
+ public:
+  Populate() = default;
+  Populate(const Populate&) = delete;
+  Populate& operator=(const Populate&) = delete;
+  ~Populate() { join(); }
+
+  // Starts on [p, p + bytes) unless it is small, or memory that the CUDA
+  // driver owns (pinned, managed).
+  void start(void* p, size_t bytes) {
+    if (!p || bytes < ((size_t)4 << 20)) return;
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+      cudaGetLastError();
+      return;
+    }
+    if (at.type != cudaMemoryTypeUnregistered) return;
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    const uintptr_t lo = ((uintptr_t)p + page - 1) / page * page;
+    const uintptr_t hi = ((uintptr_t)p + bytes) / page * page;
+    if (hi <= lo) return;
+    const size_t pages = (hi - lo) / page;
+    const unsigned hw = std::thread::hardware_concurrency();
+    const size_t n = std::max<size_t>(1, std::min<size_t>(8, hw / 2));
+    try {
+      for (size_t k = 0; k < n; ++k) {
+        const uintptr_t a = lo + pages * k / n * page, b = lo + pages * (k + 1) / n * page;
+        workers_.emplace_back([a, b] {
+          // in 8 MB steps: the address space lock is not held for long
+          for (uintptr_t q = a; q < b; q += (uintptr_t)8 << 20)
+            if (madvise((void*)q, std::min<uintptr_t>((uintptr_t)8 << 20, b - q),
+                        MADV_POPULATE_WRITE) != 0)
+              return;
+        });
+      }
+    } catch (const std::system_error&) {
+      // fewer threads, or none: the copy faults the pages in itself
+    }
+  }
+
+  void join() {
+    for (auto& t : workers_) t.join();
+    workers_.clear();
+  }
+
+ private:
+  std::vector<std::thread> workers_;
+};
+
+}  // namespace vti
