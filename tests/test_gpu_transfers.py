@@ -40,3 +40,21 @@ def test_host_and_device_arrays_agree(ctx, nx, ny, nz):
         plan.close()
     assert np.abs(res[0][1:]).max() > 0
     assert np.array_equal(res[0], res[1])
+
+
+@pytest.mark.parametrize("nt", [5, 40])
+def test_product_with_blocks_longer_than_the_record(ctx, nt):
+    """Checkpoint blocks longer than the record hold only its levels: one block
+    either way, the same sums."""
+    s = S.small3d(nx=40, ny=36, nz=32, nt=nt, npad=8, rate=2.1e-3)
+    n = s.nxyz
+    c = s.cij()
+    dc = (0.02 * c).astype(np.float32)
+    dobs = np.zeros(V.nnt3d(s.geom()) * (s.recloc.size // 4), dtype=np.float32)
+    out = [V.gnhv_exact(ctx, s.geom(), *c.reshape(3, n), s.wavelet, s.souloc, s.recloc, dc=dc,
+                        dobs=dobs, checkpoint_every=k, flags=f) for k in (nt, 64, 500)
+           for f in (0,)]
+    assert np.abs(out[0]["hv"]).max() > 0
+    for o in out[1:]:
+        for k in ("hv", "grad", "traces", "born"):
+            assert np.array_equal(o[k], out[0][k]), k

@@ -775,42 +775,41 @@ struct GnState {
   VolM ring[3][2];            // BF16 mode: FP32 levels of the recomputation
   std::vector<VolB> segb;     // BF16 mode: (K+1) levels x (x, z)
   float* damp = nullptr;
+  // Every volume and table above lies in one allocation: 221 separate ones (a
+  // 200x180x120 product of 299 levels) cost 135 ms per call in cudaMalloc and
+  // cudaFree, one of the same 4 GB costs 4.
+  char* slab = nullptr;
+  size_t slab_bytes = 0, slab_used = 0;
   ~GnState() {
-    for (auto& x : segb) {
-      if (x.alloc) cudaFree(x.alloc);
-      if (x.scale) cudaFree(x.scale);
-    }
-    for (auto& r : ring) for (auto& x : r) vol_free(&x.v);
-    for (auto& i : master)
-      for (float* q : i)
-        if (q) cudaFree(q);
-    for (auto& i : comp)
-      for (float* q : i)
-        if (q) cudaFree(q);
-    auto fr = [](VolM& x) { vol_free(&x.v); };
-    for (auto& x : c) fr(x);
-    for (auto& x : dc) fr(x);
-    for (auto& r : a) for (auto& x : r) fr(x);
-    for (auto& r : b) for (auto& x : r) fr(x);
-    for (auto& x : ck) fr(x);
-    for (auto& x : seg) fr(x);
-    for (auto& i : mu) for (auto& r : i) for (auto& x : r) fr(x);
-    for (auto& i : w) for (auto& r : i) for (auto& x : r) fr(x);
-    for (auto& i : img) for (auto& x : i) fr(x);
-    if (damp) cudaFree(damp);
+    if (slab) cudaFree(slab);
+  }
+  static size_t padded(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
+  size_t vol_bytes() const { return (size_t)d.plane * (d.nz + 2 * kZPad) * sizeof(float); }
+  // One allocation for `vols` volumes, `vols16` BF16 volumes with their scales
+  // and `flat` further bytes, cleared.
+  int reserve(size_t vols, size_t vols16, size_t flat) {
+    slab_bytes = vols * padded(vol_bytes()) +
+                 vols16 * (padded(vol_bytes() / 2) + padded((d.nz + 2 * kZPad) * sizeof(float))) +
+                 flat;
+    VTI_CUDA(ctx, cudaMalloc((void**)&slab, slab_bytes));
+    VTI_CUDA(ctx, cudaMemsetAsync(slab, 0, slab_bytes, ctx->stream));
+    return VTI_OK;
+  }
+  int take(void** out, size_t bytes) {
+    if (slab_used + padded(bytes) > slab_bytes) return fail(ctx, VTI_ERR_OOM, "Gauss-Newton slab");
+    *out = slab + slab_used;
+    slab_used += padded(bytes);
+    return VTI_OK;
   }
   int alloc(VolM* x) {
-    VTI_TRY(vol_alloc(ctx, d, &x->v));
-    VTI_TRY(vol_zero(ctx, d, &x->v));
+    VTI_TRY(take((void**)&x->v.alloc, vol_bytes()));
+    x->v.bytes = vol_bytes();
+    x->v.origin = x->v.alloc + (size_t)kZPad * d.plane;
     return make_tile_maps(ctx, d, x->v, &x->m);
   }
   int alloc(VolB* x) {
-    const size_t n = (size_t)d.plane * (d.nz + 2 * kZPad);
-    if (cudaMalloc(&x->alloc, n * 2) != cudaSuccess ||
-        cudaMalloc((void**)&x->scale, (d.nz + 2 * kZPad) * sizeof(float)) != cudaSuccess)
-      return fail(ctx, VTI_ERR_OOM, "BF16 segment");
-    VTI_CUDA(ctx, cudaMemsetAsync(x->alloc, 0, n * 2, ctx->stream));
-    VTI_CUDA(ctx, cudaMemsetAsync(x->scale, 0, (d.nz + 2 * kZPad) * sizeof(float), ctx->stream));
+    VTI_TRY(take(&x->alloc, vol_bytes() / 2));
+    VTI_TRY(take((void**)&x->scale, (d.nz + 2 * kZPad) * sizeof(float)));
     x->origin = (__nv_bfloat16*)x->alloc + (size_t)kZPad * d.plane;
     return make_tile_maps_typed(ctx, d, x->alloc, 2, &x->m);
   }
@@ -998,7 +997,7 @@ int vti3d_gnhv_exact(vti_ctx* ctx, const vti3d_geom* g, const float* c11, const 
   const unsigned flags = VTI_OPT_FULL_STEPS;
   // the per-shot helpers of the plan: receivers, schedule, damping tables
   vti3d_plan* p = nullptr;
-  VTI_TRY(vti3d_plan_create(ctx, g, flags, &p));
+  VTI_TRY(p3d::plan_tables(ctx, g, flags, &p));
   struct PlanGuard {
     vti3d_plan* p;
     ~PlanGuard() { vti3d_plan_destroy(p); }
@@ -1021,10 +1020,17 @@ int vti3d_gnhv_exact(vti_ctx* ctx, const vti3d_geom* g, const float* c11, const 
   const float dt2 = g->dt * g->dt;
   const bool want_born = hv || born;
   const bool want_grad = grad || misfit;
-  S.damp = nullptr;
-  VTI_CUDA(ctx, cudaMalloc((void**)&S.damp, p->h_damp.size() * sizeof(float)));
-  VTI_CUDA(ctx, cudaMemcpy(S.damp, p->h_damp.data(), p->h_damp.size() * sizeof(float),
-                           cudaMemcpyHostToDevice));
+  S.damp = p->dampx;
+  // checkpoints: blocks of K levels a_{1+iK} ... ; block i needs a_{iK}, a_{1+iK}
+  const int nblk = (M - 1 + K - 1) / K;
+  const int nseg = std::min(K, M - 1) + 1;  // levels of the longest block and the one before
+  // ---- device memory: model, perturbation, background and Born fields,
+  // checkpoints, segment (BF16: and its FP32 ring), per image two adjoint
+  // fields on two levels, three images and their compensated sums
+  const int nimages = (grad ? 1 : 0) + (hv ? 1 : 0);
+  const size_t plane_bytes = (size_t)S.d.plane * S.d.nz * sizeof(float);
+  VTI_TRY(S.reserve(14 + 4 * (size_t)nblk + (b16 ? 6 : 2 * (size_t)nseg) + 11 * (size_t)nimages,
+                    b16 ? 2 * (size_t)nseg : 0, 6 * (size_t)nimages * S.padded(plane_bytes)));
   const float* cs[3] = {c11, c13, c33};
   for (int k = 0; k < 3; ++k) {
     VTI_TRY(S.alloc(&S.c[k]));
@@ -1037,17 +1043,15 @@ int vti3d_gnhv_exact(vti_ctx* ctx, const vti3d_geom* g, const float* c11, const 
       VTI_TRY(S.alloc(&S.a[bf][f]));
       VTI_TRY(S.alloc(&S.b[bf][f]));
     }
-  // checkpoints: blocks of K levels a_{1+iK} ... ; block i needs a_{iK}, a_{1+iK}
-  const int nblk = (M - 1 + K - 1) / K;
   S.ck.resize(4 * (size_t)nblk);
-  for (auto& x : S.ck) VTI_TRY(vol_alloc(ctx, S.d, &x.v));
+  for (auto& x : S.ck) VTI_TRY(S.alloc(&x));
   if (b16) {
     for (auto& r : S.ring)
       for (auto& x : r) VTI_TRY(S.alloc(&x));
-    S.segb.resize(2 * (size_t)(K + 1));
+    S.segb.resize(2 * (size_t)nseg);
     for (auto& x : S.segb) VTI_TRY(S.alloc(&x));
   } else {
-    S.seg.resize(2 * (size_t)(K + 1));
+    S.seg.resize(2 * (size_t)nseg);
     for (auto& x : S.seg) VTI_TRY(S.alloc(&x));
   }
   // traces: background, Born
@@ -1121,11 +1125,8 @@ int vti3d_gnhv_exact(vti_ctx* ctx, const vti3d_geom* g, const float* c11, const 
       }
     for (int k = 0; k < 3; ++k) {
       VTI_TRY(S.alloc(&S.img[im][k]));
-      const size_t nb = (size_t)S.d.plane * S.d.nz * sizeof(float);
-      VTI_CUDA(ctx, cudaMalloc((void**)&S.master[im][k], nb));
-      VTI_CUDA(ctx, cudaMalloc((void**)&S.comp[im][k], nb));
-      VTI_CUDA(ctx, cudaMemsetAsync(S.master[im][k], 0, nb, ctx->stream));
-      VTI_CUDA(ctx, cudaMemsetAsync(S.comp[im][k], 0, nb, ctx->stream));
+      VTI_TRY(S.take((void**)&S.master[im][k], plane_bytes));
+      VTI_TRY(S.take((void**)&S.comp[im][k], plane_bytes));
     }
   }
   const long long nimg = S.d.plane * S.d.nz;

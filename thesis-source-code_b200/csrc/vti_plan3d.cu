@@ -351,6 +351,35 @@ int check_geom(vti_ctx* ctx, const vti3d_geom* g) {
   return VTI_OK;
 }
 
+int plan_tables(vti_ctx* ctx, const vti3d_geom* g, unsigned flags, vti3d_plan** out) {
+  if (!ctx || !out) return VTI_ERR_ARG;
+  *out = nullptr;
+  VTI_TRY(check_geom(ctx, g));
+  VTI_CUDA(ctx, cudaSetDevice(ctx->device));
+  vti3d_plan* p = new vti3d_plan();
+  p->ctx = ctx;
+  p->g = *g;
+  p->flags = flags;
+  p->d = make_dims(g->nx, g->ny, g->nz);
+  p->h_damp.resize((size_t)g->nx + g->ny + g->nz);
+  for (int i = 0; i < g->nx; ++i) p->h_damp[i] = damp_profile(i, g->nx, g->npad);
+  for (int i = 0; i < g->ny; ++i) p->h_damp[g->nx + i] = damp_profile(i, g->ny, g->npad);
+  for (int i = 0; i < g->nz; ++i) p->h_damp[g->nx + g->ny + i] = damp_profile(i, g->nz, g->npad);
+  cudaError_t e = cudaMalloc((void**)&p->dampx, p->h_damp.size() * sizeof(float));
+  if (e == cudaSuccess)
+    e = cudaMemcpy(p->dampx, p->h_damp.data(), p->h_damp.size() * sizeof(float),
+                   cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) {
+    const int st = cuda_check(ctx, e, "damping tables");
+    vti3d_plan_destroy(p);
+    return st;
+  }
+  p->dampy = p->dampx + g->nx;
+  p->dampz = p->dampy + g->ny;
+  *out = p;
+  return VTI_OK;
+}
+
 int get_obs(vti3d_plan* p, const ShotGeom& s, const float* dobs, int mem, const float** out) {
   const int nnt = nnt_of(p->g);
   const size_t n = (size_t)nnt * s.nr;
@@ -506,15 +535,10 @@ int vti_ctx_set_plan_cache(vti_ctx* ctx, int enable) {
 }
 
 int vti3d_plan_create(vti_ctx* ctx, const vti3d_geom* g, unsigned flags, vti3d_plan** out) {
-  if (!ctx || !out) return VTI_ERR_ARG;
+  if (!out) return VTI_ERR_ARG;
   *out = nullptr;
-  VTI_TRY(check_geom(ctx, g));
-  VTI_CUDA(ctx, cudaSetDevice(ctx->device));
-  vti3d_plan* p = new vti3d_plan();
-  p->ctx = ctx;
-  p->g = *g;
-  p->flags = flags;
-  p->d = make_dims(g->nx, g->ny, g->nz);
+  vti3d_plan* p = nullptr;
+  VTI_TRY(plan_tables(ctx, g, flags, &p));
   int st = VTI_OK;
   Vol* vols[] = {&p->cpad[0], &p->cpad[1], &p->cpad[2], &p->sx[0], &p->sx[1], &p->sz[0],
                  &p->sz[1],   &p->lx[0],   &p->lx[1],   &p->lz[0], &p->lz[1], &p->g11,
@@ -532,19 +556,6 @@ int vti3d_plan_create(vti_ctx* ctx, const vti3d_geom* g, unsigned flags, vti3d_p
     if (st == VTI_OK) st = make_tile_maps(ctx, p->d, p->g11, &p->m_g[0]);
     if (st == VTI_OK) st = make_tile_maps(ctx, p->d, p->g13, &p->m_g[1]);
     if (st == VTI_OK) st = make_tile_maps(ctx, p->d, p->g33, &p->m_g[2]);
-  }
-  if (st == VTI_OK) {
-    p->h_damp.resize((size_t)g->nx + g->ny + g->nz);
-    for (int i = 0; i < g->nx; ++i) p->h_damp[i] = damp_profile(i, g->nx, g->npad);
-    for (int i = 0; i < g->ny; ++i) p->h_damp[g->nx + i] = damp_profile(i, g->ny, g->npad);
-    for (int i = 0; i < g->nz; ++i) p->h_damp[g->nx + g->ny + i] = damp_profile(i, g->nz, g->npad);
-    cudaError_t e = cudaMalloc((void**)&p->dampx, p->h_damp.size() * sizeof(float));
-    if (e == cudaSuccess)
-      e = cudaMemcpy(p->dampx, p->h_damp.data(), p->h_damp.size() * sizeof(float),
-                     cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) st = cuda_check(ctx, e, "damping tables");
-    p->dampy = p->dampx + g->nx;
-    p->dampz = p->dampy + g->ny;
   }
   if (st != VTI_OK) {
     vti3d_plan_destroy(p);

@@ -87,6 +87,9 @@ int last_level(const vti3d_geom& g, unsigned flags);
 long long boundary_count(const vti3d_geom& g);
 float damp_profile(int i, int n, int npad);
 int check_geom(vti_ctx* ctx, const vti3d_geom* g);
+// A plan of geometry g without its volumes: grid, damping tables and the
+// per-shot helpers below.
+int plan_tables(vti_ctx* ctx, const vti3d_geom* g, unsigned flags, vti3d_plan** out);
 // Source, receivers and record schedule of shot `is` of souloc (5 floats per
 // shot) in the plan's grid.
 int shot_geom(vti3d_plan* p, const float* souloc, int is, ShotGeom* s);
