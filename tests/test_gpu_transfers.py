@@ -42,6 +42,29 @@ def test_host_and_device_arrays_agree(ctx, nx, ny, nz):
     assert np.array_equal(res[0], res[1])
 
 
+# 6 to 16 backward levels: fewer than, exactly and just over the eight summed at
+# a time; lag ranges that are not a multiple of four; odd row lengths
+@pytest.mark.parametrize("nt,nx", [(8, 40), (10, 41), (11, 47), (18, 38)])
+def test_gathers_do_not_depend_on_the_lag_range(ctx, nt, nx):
+    s = S.small3d(nx=nx, ny=24, nz=22, nt=nt, npad=5, rate=2.1e-3)
+    plan = V.Plan3d(ctx, s.geom(), V.OPT_FULL_STEPS)
+    plan.set_model(*s.cij().reshape(3, s.nxyz))
+    plan.set_wavelet(s.wavelet)
+    plan.set_receivers(s.recloc)
+    data = np.random.default_rng(1).standard_normal(
+        V.nnt3d(s.geom()) * (s.recloc.size // 4)).astype(np.float32)
+    im = plan.rtm(s.souloc, [0], data).reshape(22, 24, nx)
+    ref = plan.odcig(s.souloc, [0], data, 13).reshape(27, 22, 24, nx)
+    assert np.abs(ref).max() > 0
+    for nlag in (0, 1, 3, 4, 6):
+        g = plan.odcig(s.souloc, [0], data, nlag).reshape(2 * nlag + 1, 22, 24, nx)
+        assert np.array_equal(g[:, :, :, 13:nx - 13], ref[13 - nlag:14 + nlag, :, :, 13:nx - 13])
+        lo = max(4, nlag)
+        assert np.array_equal(g[nlag][:, :, lo:nx - lo], im[:, :, lo:nx - lo])
+        assert not g[:, :, :, :lo].any() and not g[:, :, :, nx - lo:].any()
+    plan.close()
+
+
 @pytest.mark.parametrize("nt", [5, 40])
 def test_product_with_blocks_longer_than_the_record(ctx, nt):
     """Checkpoint blocks longer than the record hold only its levels: one block

@@ -224,7 +224,8 @@ int launch_fwd3d_tma(vti_ctx* ctx, const Dims3& d, const TileMaps& cx, const Til
                      bool up = false);
 // Fused backward step: sigma back one level (gradient form, no sponge, +src),
 // adjoint lambda one level (forward form, sponge), zero-lag imaging into g
-// (rtm: the RTM image in g11 instead).
+// (rtm: the RTM image in g11 instead; with es / er also its two factors of
+// this level, plane 0 first).
 int launch_bwd3d_tma(vti_ctx* ctx, const Dims3& d, const TileMaps& scx, const TileMaps& scz,
                      const TileMaps& spx, const TileMaps& spz, const TileMaps& lcx,
                      const TileMaps& lcz, const TileMaps& lpx, const TileMaps& lpz,
@@ -233,7 +234,8 @@ int launch_bwd3d_tma(vti_ctx* ctx, const Dims3& d, const TileMaps& scx, const Ti
                      const float* scz_ptr, const float* lcz_ptr, float* spx_ptr, float* spz_ptr,
                      float* lpx_ptr, float* lpz_ptr, float* g11_ptr, float* g13_ptr,
                      float* g33_ptr, const Damping& damp, float dt2, float idx2, float idy2,
-                     float idz2, float sx, float sy, float sz, PointSource src, bool rtm, bool up = false);
+                     float idz2, float sx, float sy, float sz, PointSource src, bool rtm, bool up = false,
+                     float* es = nullptr, float* er = nullptr);
 
 // One job of a batched forward launch (k_fwd3d_tma over the items of many
 // volumes). Step s = tick - t0 of the job uses parity p = s & 1:
@@ -321,12 +323,13 @@ inline bool receivers_early(const Dims3& d, int bytes_per_point) {
 int launch_seed_adjoint(vti_ctx* ctx, float* lx, float* lz, const float* res, int nnt,
                         const long long* rec, const float* rec_damp, int nr, float dt2);
 int launch_set_point(vti_ctx* ctx, float* a, float* b, long long off, float value);
-// Offset-domain gathers of one backward level: image holds 2*nlag+1 volumes
-// of d.plane*d.nz floats (pitched rows, no z pad planes), lag -nlag first;
-// sx, sz, lx, lz are the level's current source and receiver wavefields.
-int launch_odcig3d(vti_ctx* ctx, const Dims3& d, const float* sx, const float* sz,
-                   const float* lx, const float* lz, const Damping& damp, int nlag,
-                   float* image);
+// Offset-domain gathers of nk <= kOdcigSlots backward levels: image holds
+// 2*nlag+1 volumes of d.plane*d.nz floats (pitched rows, no z pad planes), lag
+// -nlag first; level k's S and R (the RTM step's image pair, stored by
+// launch_bwd3d_tma) start at S + k*slot_stride and R + k*slot_stride.
+constexpr int kOdcigSlots = 8;
+int launch_odcig3d(vti_ctx* ctx, const Dims3& d, const float* S, const float* R,
+                   long long slot_stride, int nk, int nlag, float* image);
 // res <- modeled - observed (dead receivers: modeled zeroed first);
 // acc[0] += sum(res^2) in FP64, reproducibly; acc must hold
 // 1 + residual_blocks(ctx) doubles. obs == nullptr: only zero dead traces.

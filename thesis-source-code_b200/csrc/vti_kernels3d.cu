@@ -221,60 +221,100 @@ __global__ void k_boundary_merge(Dims3 d, int npad, const float* full, const flo
   }
 }
 
-// Offset-domain image gathers of one backward level (extendedImagingKernel,
-// lib/vti-fwi-3d/gpu/wave3d.cu:1299-1313, on this library's RTM pair): with
-// S(p) = 2/3 sx + 1/3 sz and R(p) = sponge(p) (2/3 lx + 1/3 lz) at the step's
-// current level, evaluated with the operations of the zero-lag image of the
-// fused backward kernel, image[lag][p] = fma(S(p), R(p + lag), image[lag][p])
-// for |lag| <= nlag (x offsets) and x in [xlo, xhi). One block: 128 points
-// of one row; R of the row segment and its nlag-wide margins staged in
-// shared memory.
-constexpr int kOdcigTX = 128;
-constexpr float kTwoThirdF = (float)kTwoThird, kOneThirdF = (float)kOneThird;
+// Offset-domain image gathers of up to kOdcigSlots backward levels
+// (extendedImagingKernel, lib/vti-fwi-3d/gpu/wave3d.cu:1299-1313, on this
+// library's RTM pair). The RTM step stores, per level k, S(p) = 2/3 sx + 1/3 sz
+// and R(p) = sponge(p) (2/3 lx + 1/3 lz); here image[lag][p] =
+// fma(S_k(p), R_k(p + lag), image[lag][p]) for k = 0, 1, .. in level order,
+// |lag| <= nlag (x offsets) and x in [xlo, xhi).
+//
+// Bound by the image traffic, 8 bytes per point and lag (65 lags: 520 bytes per
+// point): summing eight levels per pass divides it by eight, for 16 bytes per
+// point and level of S and R. A thread owns four consecutive points and takes
+// the lags four at a time: sixteen FMAs per level on one new float4 of R (the
+// row is reused from L1) and one float4 of the image per lag.
+// 150x120x80, 32 lags each side: 156 us per level for the one-level kernel,
+// 31 us per level for this one.
+__device__ __forceinline__ float4 odcig_row4(const float* row, int x, int pitch) {
+  return x >= 0 && x < pitch ? __ldg(reinterpret_cast<const float4*>(row + x))
+                             : make_float4(0.f, 0.f, 0.f, 0.f);
+}
 
-__global__ void __launch_bounds__(kOdcigTX)
-    k_odcig3d(Dims3 d, const float* sx, const float* sz, const float* lx, const float* lz,
-              const float* dampx, const float* dampy, const float* dampz, int nlag, int xlo,
-              int xhi, float* image, long long lag_stride) {
-  extern __shared__ float rs[];  // R at x0 - nlag .. x0 + kOdcigTX + nlag - 1
-  const int x0 = blockIdx.x * kOdcigTX;
-  const int y = kHalo + blockIdx.y;
-  const int z = blockIdx.z;
-  const float dz = dampz[z], dy = dampy[y];
+__global__ void __launch_bounds__(128)
+    k_odcig3d(Dims3 d, const float* S, const float* R, long long slot_stride, int nk, int nlag,
+              int xlo, int xhi, float* image, long long lag_stride) {
+  const int groups = (xhi + 3) / 4;  // float4 groups of a row that hold updated points
+  const long long rows = (long long)(d.ny - 2 * kHalo) * d.nz;
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t >= rows * groups) return;
+  const long long rw = t / groups;
+  const int x = 4 * (int)(t - rw * groups);
+  if (x + 3 < xlo) return;
+  const int y = kHalo + (int)(rw % (d.ny - 2 * kHalo)), z = (int)(rw / (d.ny - 2 * kHalo));
   const long long row = (long long)z * d.plane + (long long)y * d.pitch;
-  for (int t = threadIdx.x; t < kOdcigTX + 2 * nlag; t += kOdcigTX) {
-    const int xr = x0 - nlag + t;
-    float r = 0.f;
-    if (xr >= 0 && xr < d.nx) {
-      const float dd = (dampx[xr] * dy) * dz;
-      r = dd * fmaf(kTwoThirdF, lx[row + xr], kOneThirdF * lz[row + xr]);
-    }
-    rs[t] = r;
+  const int lag0 = -((nlag + 3) & ~3);  // aligned start; lags below -nlag are skipped
+  float s[kOdcigSlots][4];
+  float4 hi[kOdcigSlots];
+#pragma unroll
+  for (int k = 0; k < kOdcigSlots; ++k) {
+    const float4 v = k < nk ? odcig_row4(S + k * slot_stride + row, x, d.pitch)
+                            : make_float4(0.f, 0.f, 0.f, 0.f);
+    s[k][0] = v.x;
+    s[k][1] = v.y;
+    s[k][2] = v.z;
+    s[k][3] = v.w;
+    hi[k] = k < nk ? odcig_row4(R + k * slot_stride + row, x + lag0, d.pitch)
+                   : make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  __syncthreads();
-  const int x = x0 + threadIdx.x;
-  if (x < xlo || x >= xhi) return;
-  const float sv = fmaf(kTwoThirdF, sx[row + x], kOneThirdF * sz[row + x]);
-  float* img = image + row + x;
-  for (int lag = -nlag; lag <= nlag; ++lag) {
-    float* q = img + (long long)(lag + nlag) * lag_stride;
-    *q = fmaf(sv, rs[threadIdx.x + nlag + lag], *q);
+  const bool full = x >= xlo && x + 3 < xhi;
+  for (int lag = lag0; lag <= nlag; lag += 4) {
+    float4 a[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const bool on = lag + j >= -nlag && lag + j <= nlag;
+      a[j] = on ? *reinterpret_cast<const float4*>(image + (lag + j + nlag) * lag_stride + row + x)
+                : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int k = 0; k < kOdcigSlots; ++k) {
+      if (k >= nk) break;
+      const float4 lo = hi[k];
+      hi[k] = odcig_row4(R + k * slot_stride + row, x + lag + 4, d.pitch);
+      const float w[7] = {lo.x, lo.y, lo.z, lo.w, hi[k].x, hi[k].y, hi[k].z};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        a[j].x = fmaf(s[k][0], w[j], a[j].x);
+        a[j].y = fmaf(s[k][1], w[j + 1], a[j].y);
+        a[j].z = fmaf(s[k][2], w[j + 2], a[j].z);
+        a[j].w = fmaf(s[k][3], w[j + 3], a[j].w);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (lag + j < -nlag || lag + j > nlag) continue;
+      float* q = image + (lag + j + nlag) * lag_stride + row + x;
+      if (full) {
+        *reinterpret_cast<float4*>(q) = a[j];
+      } else {
+        const float v[4] = {a[j].x, a[j].y, a[j].z, a[j].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (x + e >= xlo && x + e < xhi) q[e] = v[e];
+      }
+    }
   }
 }
 
 }  // namespace
 
-int launch_odcig3d(vti_ctx* ctx, const Dims3& d, const float* sx, const float* sz,
-                   const float* lx, const float* lz, const Damping& damp, int nlag,
-                   float* image) {
+int launch_odcig3d(vti_ctx* ctx, const Dims3& d, const float* S, const float* R,
+                   long long slot_stride, int nk, int nlag, float* image) {
   const int xlo = nlag > kHalo ? nlag : kHalo;
   const int xhi = d.nx - xlo;
-  if (xhi <= xlo || d.ny <= 2 * kHalo || d.nz < 1) return VTI_OK;
-  dim3 grid((d.nx + kOdcigTX - 1) / kOdcigTX, d.ny - 2 * kHalo, d.nz);
-  const size_t smem = (kOdcigTX + 2 * (size_t)nlag) * sizeof(float);
-  k_odcig3d<<<grid, kOdcigTX, smem, ctx->stream>>>(d, sx, sz, lx, lz, damp.x, damp.y, damp.z,
-                                                   nlag, xlo, xhi, image,
-                                                   d.plane * (long long)d.nz);
+  if (xhi <= xlo || d.ny <= 2 * kHalo || d.nz < 1 || nk < 1) return VTI_OK;
+  const long long threads = (long long)(d.ny - 2 * kHalo) * d.nz * ((xhi + 3) / 4);
+  k_odcig3d<<<(unsigned)((threads + 127) / 128), 128, 0, ctx->stream>>>(
+      d, S, R, slot_stride, nk, nlag, xlo, xhi, image, d.plane * (long long)d.nz);
   VTI_LAUNCHED(ctx, "k_odcig3d");
   return VTI_OK;
 }

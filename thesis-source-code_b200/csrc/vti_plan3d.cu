@@ -267,7 +267,7 @@ int forward_pass(vti3d_plan* p, const ShotGeom& s, bool sponge) {
 // added into g11/g13/g33 (the RTM image into g11), then the residual of time
 // nt-2-i injected into the new adjoint level (injectRecord3d.cu:60-78).
 int bwd_level(vti3d_plan* p, const ShotGeom& s, bool rtm, int SA, int SB, int LA, int LB,
-              int i) {
+              int i, float* es, float* er) {
   vti_ctx* ctx = p->ctx;
   const vti3d_geom& g = p->g;
   const float dx2 = g.dx * g.dx, dy2 = g.dy * g.dy, dz2 = g.dz * g.dz, dt2 = g.dt * g.dt;
@@ -286,7 +286,7 @@ int bwd_level(vti3d_plan* p, const ShotGeom& s, bool rtm, int SA, int SB, int LA
       p->sz[SA].origin, p->lz[LA].origin, p->sx[SB].origin, p->sz[SB].origin,
       p->lx[LB].origin, p->lz[LB].origin, p->g11.origin, p->g13.origin, p->g33.origin, dmp,
       dt2, 1.f / dx2, 1.f / dy2, 1.f / dz2, dt2 / dx2, dt2 / dy2, dt2 / dz2, src, rtm,
-      (i & 1) != 0));
+      (i & 1) != 0, es, er));
   // residual interpolated at it+1 (injectRecord3d.cu:60-78)
   const int ti = it + 1;
   float f = float(ti) / float(st);
@@ -303,16 +303,15 @@ int bwd_level(vti3d_plan* p, const ShotGeom& s, bool rtm, int SA, int SB, int LA
 // sx[other] = level M-1 from pass 2, and the residual in d_trace.
 // rtm: the observed traces are in d_trace and the RTM image accumulates in
 // g11 (rtm3d_f.cu:470-620, same schedule).
-// ext (nlag >= 0, RTM only): offset-domain gathers of each level added after
-// its fused step, from the same current wavefields.
-int backward_pass(vti3d_plan* p, const ShotGeom& s, bool rtm, float* ext, int nlag) {
+// ext (RTM only): offset-domain gathers, summed whenever the slots of S and R
+// are full, in level order.
+int backward_pass(vti3d_plan* p, const ShotGeom& s, bool rtm, const Gathers* ext) {
   NvtxRange nv(rtm ? "vti3d RTM back-propagation" : "vti3d pass 3 (reconstruction, adjoint, imaging)");
   vti_ctx* ctx = p->ctx;
   const vti3d_geom& g = p->g;
   const Dims3& d = p->d;
   const float dt2 = g.dt * g.dt;
   const int nnt = nnt_of(g), M = last_level(g, p->flags);
-  Damping dmp{p->dampx, p->dampy, p->dampz};
   // flip (objFuncGradient3d_f.cu:912-914): cur = level M-1, prev = level M
   int SA = 1 - p->last_cur, SB = p->last_cur;
   for (int k = 0; k < 2; ++k) {
@@ -323,12 +322,13 @@ int backward_pass(vti3d_plan* p, const ShotGeom& s, bool rtm, float* ext, int nl
   VTI_TRY(launch_seed_adjoint(ctx, p->lx[LA].origin, p->lz[LA].origin, p->d_trace, nnt,
                               p->d_rec + p->rec_cap, p->d_rec_damp, s.nr, dt2));
   for (int i = 0; i < M - 1; ++i) {
-    VTI_TRY(bwd_level(p, s, rtm, SA, SB, LA, LB, i));
-    // the gathers read the current levels sx[SA], lx[LA]; the step and the
-    // injection write only sx[SB], lx[LB]
-    if (ext)
-      VTI_TRY(launch_odcig3d(ctx, d, p->sx[SA].origin, p->sz[SA].origin, p->lx[LA].origin,
-                             p->lz[LA].origin, dmp, nlag, ext));
+    const int slot = ext ? i % ext->slots : 0;
+    VTI_TRY(bwd_level(p, s, rtm, SA, SB, LA, LB, i,
+                      ext ? ext->S + slot * ext->slot_stride : nullptr,
+                      ext ? ext->R + slot * ext->slot_stride : nullptr));
+    if (ext && (slot + 1 == ext->slots || i + 1 == M - 1))
+      VTI_TRY(launch_odcig3d(ctx, d, ext->S, ext->R, ext->slot_stride, slot + 1, ext->nlag,
+                             ext->image));
     std::swap(SA, SB);
     std::swap(LA, LB);
   }
@@ -583,7 +583,7 @@ int vti3d_plan_destroy(vti3d_plan* p) {
   vol_free(&p->g13);
   vol_free(&p->g33);
   void* ptrs[] = {p->dampx, p->d_rec, p->d_rec_damp, p->d_live, p->d_trace,
-                  p->d_obs, p->d_blist, p->d_acc, p->d_gw, p->d_part, p->d_ext,
+                  p->d_obs, p->d_blist, p->d_acc, p->d_gw, p->d_part, p->d_ext, p->d_exf,
                   p->d_obs16, p->d_obs_scale};
   for (void* q : ptrs)
     if (q) cudaFree(q);
@@ -797,6 +797,22 @@ int vti3d_plan_odcig(vti3d_plan* p, const float* souloc, const int* shotid, int 
   VTI_CUDA(ctx, cudaMemsetAsync(p->d_ext, 0, nl * vol * sizeof(float), ctx->stream));
   // the zero-lag image of the same passes accumulates in g11 (unused here)
   VTI_TRY(vol_zero(ctx, d, &p->g11));
+  // S and R of kOdcigSlots levels, or of one in g13 and g33 (the RTM step leaves
+  // them alone) when the device has no room; zero in the frame the step skips
+  Gathers ext{p->d_ext, nullptr, nullptr, (long long)vol, kOdcigSlots, nlag};
+  const size_t nf = 2 * (size_t)kOdcigSlots * vol;
+  if (ensure(ctx, &p->d_exf, &p->exf_cap, nf) == VTI_OK) {
+    VTI_CUDA(ctx, cudaMemsetAsync(p->d_exf, 0, nf * sizeof(float), ctx->stream));
+    ext.S = p->d_exf;
+    ext.R = p->d_exf + kOdcigSlots * vol;
+  } else {
+    cudaGetLastError();
+    VTI_TRY(vol_zero(ctx, d, &p->g13));
+    VTI_TRY(vol_zero(ctx, d, &p->g33));
+    ext.slots = 1;
+    ext.S = p->g13.origin;
+    ext.R = p->g33.origin;
+  }
   for (int k = 0; k < nshot; ++k) {
     ShotGeom s;
     VTI_TRY(shot_geom(p, souloc, shotid[k], &s));
@@ -807,7 +823,7 @@ int vti3d_plan_odcig(vti3d_plan* p, const float* souloc, const int* shotid, int 
       VTI_CUDA(ctx, cudaMemcpyAsync(p->d_trace, obs, (size_t)nnt * s.nr * sizeof(float),
                                     cudaMemcpyDeviceToDevice, ctx->stream));
     VTI_TRY(forward_pass(p, s, false));
-    VTI_TRY(backward_pass(p, s, true, p->d_ext, nlag));
+    VTI_TRY(backward_pass(p, s, true, &ext));
     VTI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   }
   const size_t nxyz = (size_t)d.nx * d.ny * d.nz;

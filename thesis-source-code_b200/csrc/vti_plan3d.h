@@ -56,6 +56,8 @@ struct vti3d_plan {
   size_t gw_cap = 0;
   float* d_ext = nullptr;  // offset-domain gathers ((2 nlag + 1) pitched volumes)
   size_t ext_cap = 0;
+  float* d_exf = nullptr;  // their S and R slots
+  size_t exf_cap = 0;
   double* d_part = nullptr;  // per-trace AGC misfits
   size_t part_cap = 0;
   // misfit options of the gradient (objFuncGradient3d_f.cu:743-775)
@@ -105,14 +107,23 @@ int fwd_level(vti3d_plan* p, const ShotGeom& s, bool sponge, int A, int B, int i
 // Backward step i of pass 3 with its residual injection: source fields
 // sx[SA] (current) / sx[SB] (overwritten), adjoint lx[LA] / lx[LB]
 // (overwritten), imaging into g11/g13/g33.
+// es, er: see launch_bwd3d_tma.
 int bwd_level(vti3d_plan* p, const ShotGeom& s, bool rtm, int SA, int SB, int LA, int LB,
-              int i);
+              int i, float* es = nullptr, float* er = nullptr);
+// Offset-domain gathers accumulated beside an RTM pass: the image and the
+// slots that hold S and R of the levels not yet summed.
+struct Gathers {
+  float* image;
+  float* S;
+  float* R;
+  long long slot_stride;
+  int slots, nlag;
+};
 // Whole passes: forward_pass leaves level M in sx[last_cur] and M-1 in the
-// other buffer; backward_pass runs the M-1 backward steps from there (nlag
-// offset-domain gathers into ext when ext is given).
+// other buffer; backward_pass runs the M-1 backward steps from there (with
+// offset-domain gathers when ext is given).
 int forward_pass(vti3d_plan* p, const ShotGeom& s, bool sponge);
-int backward_pass(vti3d_plan* p, const ShotGeom& s, bool rtm, float* ext = nullptr,
-                  int nlag = 0);
+int backward_pass(vti3d_plan* p, const ShotGeom& s, bool rtm, const Gathers* ext = nullptr);
 
 template <typename T>
 int ensure(vti_ctx* ctx, T** ptr, size_t* cap, size_t n) {

@@ -470,6 +470,8 @@ struct BwdPar {
   float* spz;
   float* lpx;
   float* lpz;
+  float* es;         // RTM: the image's two factors stored as well, or null
+  float* er;
 };
 struct BwdArgs {
   BwdCommon c;
@@ -664,9 +666,13 @@ __device__ __forceinline__ bool bwd_consume(const BwdCommon& a, const BwdPar& bp
     const float2 lz0 = lq[4];
     const float2 dd = mul2(make_float2(dxy[0], dxy[1]), splat(dz));
     if (kRtm) {
-      store2(a.g11, fma2(fma2(splat(kTwoThirdF), sc, mul2(splat(kOneThirdF), sq[4])),
-                         mul2(dd, fma2(splat(kTwoThirdF), lc, mul2(splat(kOneThirdF), lz0))),
-                         g11o));
+      const float2 es = fma2(splat(kTwoThirdF), sc, mul2(splat(kOneThirdF), sq[4]));
+      const float2 er = mul2(dd, fma2(splat(kTwoThirdF), lc, mul2(splat(kOneThirdF), lz0)));
+      store2(a.g11, fma2(es, er, g11o));
+      if (bp.es) {
+        store2(bp.es, es);
+        store2(bp.er, er);
+      }
     } else {
       store2(a.g11, fma2(lc, sxy_u, g11o));
       store2(a.g33, fma2(lz0, sz_u, g33o));
@@ -961,7 +967,8 @@ int launch_bwd3d_tma(vti_ctx* ctx, const Dims3& d, const TileMaps& scx, const Ti
                      const float* scz_ptr, const float* lcz_ptr, float* spx_ptr, float* spz_ptr,
                      float* lpx_ptr, float* lpz_ptr, float* g11_ptr, float* g13_ptr,
                      float* g33_ptr, const Damping& damp, float dt2, float idx2, float idy2,
-                     float idz2, float sx, float sy, float sz, PointSource src, bool rtm, bool up) {
+                     float idz2, float sx, float sy, float sz, PointSource src, bool rtm, bool up,
+                     float* es, float* er) {
   void (*const kerns[4])(BwdMaps, BwdArgs) = {k_bwd3d_tma<false, 1>, k_bwd3d_tma<false, -1>,
                                               k_bwd3d_tma<true, 1>, k_bwd3d_tma<true, -1>};
   const int variant = 2 * (rtm ? 1 : 0) + (up ? 1 : 0);
@@ -980,7 +987,7 @@ int launch_bwd3d_tma(vti_ctx* ctx, const Dims3& d, const TileMaps& scx, const Ti
   c.dt2 = dt2; c.idx2 = idx2; c.idy2 = idy2; c.idz2 = idz2;
   c.sx = sx; c.sy = sy; c.sz = sz;
   c.src = src;
-  a.p = BwdPar{scz_ptr, lcz_ptr, spx_ptr, spz_ptr, lpx_ptr, lpz_ptr};
+  a.p = BwdPar{scz_ptr, lcz_ptr, spx_ptr, spz_ptr, lpx_ptr, lpz_ptr, es, er};
   a.status = ctx->d_status;
   const int grid = c.sc.grid;
   {
@@ -1095,7 +1102,7 @@ int bwd_batch_build(vti_ctx* ctx, const BwdJobSpec* spec, int njobs, StepBatch**
       c.t0 = sp.t0;
       for (int par = 0; par < 2; ++par) {
         B.p[j][par] = BwdPar{sp.scz_ptr[par], sp.lcz_ptr[par], sp.spx_ptr[par], sp.spz_ptr[par],
-                             sp.lpx_ptr[par], sp.lpz_ptr[par]};
+                             sp.lpx_ptr[par], sp.lpz_ptr[par], nullptr, nullptr};
         BwdMaps& m = maps[2 * j + par];
         m.scx = *H(*sp.scx[par]); m.scz = *P(*sp.scz[par]); m.spx = *P(*sp.spx[par]);
         m.spz = *P(*sp.spz[par]);
