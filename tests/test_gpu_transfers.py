@@ -1,5 +1,6 @@
-"""Host arrays of pitched volumes (staged, packed and unpacked on the device) against device arrays of the same calls: equal bit for
-bit."""
+"""Host arrays of pitched volumes (staged, packed and unpacked on the device,
+pages populated beforehand) against device arrays of the same calls, and the
+offset gathers summed eight levels at a time: equal bit for bit."""
 import numpy as np
 import pytest
 

@@ -36,6 +36,7 @@
 #include <cuda_bf16.h>
 
 #include "vti_plan3d.h"
+#include "vti_populate.h"
 #include "vti_tma_common.cuh"
 
 namespace vti {
@@ -1031,6 +1032,9 @@ int vti3d_gnhv_exact(vti_ctx* ctx, const vti3d_geom* g, const float* c11, const 
   const size_t plane_bytes = (size_t)S.d.plane * S.d.nz * sizeof(float);
   VTI_TRY(S.reserve(14 + 4 * (size_t)nblk + (b16 ? 6 : 2 * (size_t)nseg) + 11 * (size_t)nimages,
                     b16 ? 2 * (size_t)nseg : 0, 6 * (size_t)nimages * S.padded(plane_bytes)));
+  Populate pages;
+  for (float* o : {grad, hv})
+    pages.start(o, 3 * (size_t)S.d.npoints() * sizeof(float));
   const float* cs[3] = {c11, c13, c33};
   for (int k = 0; k < 3; ++k) {
     VTI_TRY(S.alloc(&S.c[k]));
@@ -1207,6 +1211,7 @@ int vti3d_gnhv_exact(vti_ctx* ctx, const vti3d_geom* g, const float* c11, const 
         k_unfold<<<fgrid, 256, 0, ctx->stream>>>(S.master[im][k], S.img[im][k].v.origin, nimg);
         VTI_LAUNCHED(ctx, "k_unfold");
       }
+  pages.join();
   const size_t n = (size_t)S.d.npoints();
   float* outs[2] = {grad, hv};
   for (int im = 0; im < 2; ++im)

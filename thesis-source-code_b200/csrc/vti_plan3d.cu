@@ -18,6 +18,7 @@
 #include <initializer_list>
 
 #include "vti_plan3d.h"
+#include "vti_populate.h"
 
 using namespace vti;
 using namespace vti::p3d;
@@ -430,6 +431,9 @@ int run_gradient(vti3d_plan* p, const float* souloc, const int* shotid, int nsho
   if (!p->d_acc)
     VTI_CUDA(ctx, cudaMalloc((void**)&p->d_acc, (1 + residual_blocks(ctx)) * sizeof(double)));
   VTI_CUDA(ctx, cudaMemsetAsync(p->d_acc, 0, sizeof(double), ctx->stream));
+  Populate pages;
+  if (!misfit_only && fgcij && fgcij_mem != VTI_MEM_DEVICE)
+    pages.start(fgcij, (1 + 3 * (size_t)d.npoints()) * sizeof(float));
   if (!misfit_only) {
     VTI_TRY(vol_zero(ctx, d, &p->g11));
     VTI_TRY(vol_zero(ctx, d, &p->g13));
@@ -467,6 +471,7 @@ int run_gradient(vti3d_plan* p, const float* souloc, const int* shotid, int nsho
   double acc = 0;
   VTI_CUDA(ctx, cudaMemcpyAsync(&acc, p->d_acc, sizeof(double), cudaMemcpyDeviceToHost,
                                 ctx->stream));
+  pages.join();
   if (!misfit_only && fgcij) {
     const size_t n = (size_t)d.npoints();
     VTI_TRY(vol_download(ctx, d, &p->g11, fgcij + 1, fgcij_mem));
@@ -757,6 +762,8 @@ int vti3d_plan_rtm(vti3d_plan* p, const float* souloc, const int* shotid, int ns
     return fail(ctx, VTI_ERR_ARG, "null pointer or negative shot count");
   VTI_CUDA(ctx, cudaSetDevice(ctx->device));
   const int nnt = nnt_of(p->g);
+  Populate pages;
+  if (image_mem != VTI_MEM_DEVICE) pages.start(image, (size_t)p->d.npoints() * sizeof(float));
   // rtm3d_f.cu:175: the image is zeroed, then summed over the shots
   VTI_TRY(vol_zero(ctx, p->d, &p->g11));
   for (int k = 0; k < nshot; ++k) {
@@ -774,6 +781,7 @@ int vti3d_plan_rtm(vti3d_plan* p, const float* souloc, const int* shotid, int ns
     VTI_TRY(backward_pass(p, s, true));
     VTI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   }
+  pages.join();
   VTI_TRY(vol_download(ctx, p->d, &p->g11, image, image_mem));
   VTI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return check_device_status(ctx);
@@ -793,6 +801,8 @@ int vti3d_plan_odcig(vti3d_plan* p, const float* souloc, const int* shotid, int 
   const int nnt = nnt_of(p->g);
   const int nl = 2 * nlag + 1;
   const size_t vol = (size_t)d.plane * d.nz;  // one lag: pitched rows, no pad planes
+  Populate pages;
+  if (image_mem != VTI_MEM_DEVICE) pages.start(image, nl * (size_t)d.npoints() * sizeof(float));
   VTI_TRY(ensure(ctx, &p->d_ext, &p->ext_cap, nl * vol));
   VTI_CUDA(ctx, cudaMemsetAsync(p->d_ext, 0, nl * vol * sizeof(float), ctx->stream));
   // the zero-lag image of the same passes accumulates in g11 (unused here)
@@ -826,6 +836,7 @@ int vti3d_plan_odcig(vti3d_plan* p, const float* souloc, const int* shotid, int 
     VTI_TRY(backward_pass(p, s, true, &ext));
     VTI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   }
+  pages.join();
   const size_t nxyz = (size_t)d.nx * d.ny * d.nz;
   for (int l = 0; l < nl; ++l)
     VTI_TRY(rows_download(ctx, d, p->d_ext + l * vol, image + l * nxyz, image_mem));
