@@ -102,11 +102,15 @@ uint64_t vti_ctx_kernel_launches(const vti_ctx* ctx);
  * "step2d". vti_ctx_kernel_time synchronizes the stream and returns the summed
  * device time (ms) and the number of timed launches. */
 int vti_ctx_set_timing(vti_ctx* ctx, int enable);
-/* 2D traces (vti2d_synthetic) of a grid whose state fits the shared memory of
- * one thread-block cluster (up to 16 CTAs; (nnx-8) <= 1024 columns, e.g.
+/* 2D traces (vti2d_synthetic), gradients (vti2d_gradient) and migrations
+ * (vti2d_rtm) advance several levels per launch in tiles of the grid, when
+ * sources and receivers lie in the update region and no two receivers of a shot
+ * share a cell. Traces of several shots of a grid whose state fits the shared
+ * memory of one thread-block cluster (up to 16 CTAs; (nnx-8) <= 1024 columns, e.g.
  * 461 x 261) run with the wavefields resident on chip, one cluster per shot
- * (shots with disjoint receiver ranges in one launch); results are those of
- * the per-step path. enable = 0 forces the per-step path (default 1). */
+ * (shots with disjoint receiver ranges in one launch), where that is faster.
+ * Results are those of the per-step path. enable = 0 forces the per-step path
+ * (default 1). */
 int vti_ctx_set_2d_resident(vti_ctx* ctx, int enable);
 int vti_ctx_kernel_time(vti_ctx* ctx, const char* kernel, double* total_ms, uint64_t* count);
 /* Diagnostic (no counterpart in the reference): one CTA waits on a shared-

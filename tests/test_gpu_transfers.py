@@ -76,9 +76,8 @@ def test_product_with_blocks_longer_than_the_record(ctx, nt):
     dc = (0.02 * c).astype(np.float32)
     dobs = np.zeros(V.nnt3d(s.geom()) * (s.recloc.size // 4), dtype=np.float32)
     out = [V.gnhv_exact(ctx, s.geom(), *c.reshape(3, n), s.wavelet, s.souloc, s.recloc, dc=dc,
-                        dobs=dobs, checkpoint_every=k, flags=f) for k in (nt, 64, 500)
-           for f in (0,)]
-    assert np.abs(out[0]["hv"]).max() > 0
+                        dobs=dobs, checkpoint_every=k) for k in (nt, 64, 500)]
+    assert nt == 5 or np.abs(out[0]["hv"]).max() > 0  # nothing has reached a receiver by then
     for o in out[1:]:
         for k in ("hv", "grad", "traces", "born"):
             assert np.array_equal(o[k], out[0][k]), k

@@ -185,6 +185,23 @@ int vol_download(vti_ctx* ctx, const Dims3& d, const Vol* v, float* dst, int mem
   return rows_download(ctx, d, v->origin, dst, mem);
 }
 
+// The context's 2D scratch, grown (never shrunk) to `bytes`; freed with the
+// context.
+int scratch2d(vti_ctx* ctx, size_t bytes, float** out) {
+  if (ctx->scratch2d_bytes < bytes) {
+    if (ctx->scratch2d) {
+      VTI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+      cudaFree(ctx->scratch2d);
+      ctx->scratch2d = nullptr;
+      ctx->scratch2d_bytes = 0;
+    }
+    VTI_CUDA(ctx, cudaMalloc((void**)&ctx->scratch2d, bytes));
+    ctx->scratch2d_bytes = bytes;
+  }
+  *out = ctx->scratch2d;
+  return VTI_OK;
+}
+
 int check_device_status(vti_ctx* ctx) {
   int h = 0;
   VTI_CUDA(ctx, cudaMemcpyAsync(&h, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost,

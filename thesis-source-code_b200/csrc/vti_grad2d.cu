@@ -16,6 +16,7 @@
 #include <map>
 
 #include "vti_internal.h"
+#include "vti_tile2d.h"
 
 namespace vti {
 namespace {
@@ -362,6 +363,225 @@ struct Buf {
   }
 };
 
+// The gradient through the tiled kernels (vti_tile2d.cu): receivers of a shot in
+// the update region and on different cells, sources in it as well. The same
+// levels, checkpoints and injections as run_grad2d. VTI_ERR_UNSUPPORTED: not
+// eligible, nothing was computed.
+int grad2d_tiles(vti_ctx* ctx, const vti2d_geom* g, float* gc11, float* gc13, float* gc33,
+                 const float* data, const float* c11, const float* c13, const float* c33,
+                 const float* wavelet, const int* sloc, int ns, const int* rloc, int nr,
+                 const float* taper, double* misfit, const std::vector<std::vector<Pair>>& sched,
+                 std::map<long, int>& slot, int ratio, int ntNeg, int nnt_data) {
+  const int nnx = g->nx + 2 * g->npad, nnz = g->nz + 2 * g->npad, nt = g->nt;
+  const size_t nnxz = (size_t)nnx * nnz;
+  if (!ctx->resident2d || ns < 1 || nnxz > (1u << 30)) return VTI_ERR_UNSUPPORTED;
+  int max_nri = 1;
+  for (int is = 0; is < ns; ++is) {
+    const int* sl = sloc + 4 * is;
+    if (sl[2] < 0 || sl[3] < 0 || sl[3] + sl[2] > nr || sl[0] < kHalo || sl[0] >= nnx - kHalo ||
+        sl[1] < kHalo || sl[1] >= nnz - kHalo ||
+        !tile2d::receivers_fit(nnx, nnz, rloc + 2 * sl[3], sl[2], false))
+      return VTI_ERR_UNSUPPORTED;
+    max_nri = std::max(max_nri, sl[2]);
+  }
+  const float dt = g->dt, dt2 = dt * dt;
+  const tile2d::Layout L = tile2d::make_layout(ctx, nnx, nnz, 1, true);
+  const int zero = (int)slot.size();  // one more checkpoint, of zeros
+  const size_t nrec = (size_t)nnt_data * max_nri;
+  float *flat, *model, *waves, *grad, *kept, *rec, *obs, *d_amp;
+  int *d_map, *d_row, *d_keep, *d_src, *d_nri, *d_cells;
+  long long* d_off;
+  double* d_acc;
+  unsigned char* live;
+  tile2d::BackLevel* d_lv;
+  Buf own;  // a block larger than the context keeps
+  float* block = nullptr;
+  for (int pass = 0; pass < 2; ++pass) {
+    tile2d::Carve c{reinterpret_cast<char*>(block)};
+    flat = c.take<float>(nnxz);
+    model = c.take<float>(4 * L.n);
+    waves = c.take<float>(tile2d::kWaveArrays * L.n);
+    grad = c.take<float>(3 * L.n);
+    kept = c.take<float>(2 * (size_t)(zero + 1) * L.n);
+    d_map = c.take<int>(L.n);
+    rec = c.take<float>(nrec);
+    obs = c.take<float>(nrec);
+    d_amp = c.take<float>(nt);
+    d_row = c.take<int>(nt);
+    d_keep = c.take<int>(nt);
+    d_src = c.take<int>(1);
+    d_nri = c.take<int>(1);
+    d_off = c.take<long long>(1);
+    d_cells = c.take<int>(max_nri);
+    d_acc = c.take<double>(1 + residual_blocks(ctx));
+    live = c.take<unsigned char>(nnt_data);
+    d_lv = c.take<tile2d::BackLevel>(nt);
+    if (pass) break;
+    if (c.used <= kScratch2dKeep) {
+      const int st = scratch2d(ctx, c.used, &block);
+      if (st != VTI_OK) return st;
+    } else {
+      VTI_CUDA(ctx, cudaMalloc((void**)&own.p, c.used));
+      block = own.p;
+    }
+  }
+  cudaStream_t s = ctx->stream;
+  VTI_CUDA(ctx, cudaMemsetAsync(model, 0, 4 * L.n * sizeof(float), s));
+  const float* host[4] = {c11, c13, c33, taper};
+  for (int k = 0; k < 4; ++k) {
+    VTI_CUDA(ctx, cudaMemcpyAsync(flat, host[k], nnxz * sizeof(float), cudaMemcpyHostToDevice, s));
+    const int st = tile2d::launch_pad(ctx, L, flat, model + k * L.n, true);
+    if (st != VTI_OK) return st;
+  }
+  VTI_CUDA(ctx, cudaMemsetAsync(grad, 0, 3 * L.n * sizeof(float), s));
+  VTI_CUDA(ctx, cudaMemsetAsync(kept + 2 * (size_t)zero * L.n, 0, 2 * L.n * sizeof(float), s));
+  VTI_CUDA(ctx, cudaMemsetAsync(d_acc, 0, sizeof(double), s));
+  VTI_CUDA(ctx, cudaMemsetAsync(live, 1, nnt_data, s));
+  tile2d::Forward f{};
+  f.L = L;
+  f.m = {model, model + L.n, model + 2 * L.n, model + 3 * L.n, 1.f / (g->dx * g->dx),
+         1.f / (g->dz * g->dz), dt2};
+  f.shots = 1;
+  f.src = d_src;
+  f.amp = d_amp;
+  f.rmap = d_map;
+  f.rec_row = d_row;
+  f.rec = rec;
+  f.rec_off = d_off;
+  f.nri = d_nri;
+  f.keep_mode = tile2d::kKeepD;
+  f.keep = d_keep;
+  f.kept = kept;
+  VTI_CUDA(ctx, cudaMemsetAsync(d_off, 0, sizeof(long long), s));
+  for (int is = 0; is < ns; ++is) {
+    const int* sl = sloc + 4 * is;
+    const int nri = sl[2], ir0 = sl[3], src = L.at(sl[0], sl[1]);
+    std::vector<int> cells(std::max(nri, 1)), row(nt, -1), keep(nt, -1);
+    for (int ir = 0; ir < nri; ++ir)
+      cells[ir] = L.at(rloc[2 * (ir0 + ir)], rloc[2 * (ir0 + ir) + 1]);
+    std::vector<float> amp(nt, 0.f);
+    auto find = [&](int t) {
+      const auto p = slot.find((long)is * (nt + 1) + t);
+      return p == slot.end() ? -1 : p->second;
+    };
+    for (int it = 1; it < nt; ++it) {
+      keep[it] = find(it);
+      const float t = it * dt + g->ot;
+      if (it >= 2 && t >= 0.f && (it - ntNeg) % ratio == 0 && nri > 0)
+        row[it] = (it - ntNeg) / ratio;
+      amp[it] = dt2 * wavelet[it - 1];
+    }
+    // backward levels: image pairs and injected rows (injectData)
+    const int steps = nt - 2;
+    std::vector<tile2d::BackLevel> lv(steps + 1);
+    int b0 = nnt_data - 1, b1 = -1;
+    auto slot_of = [&](long label) { return label < 0 ? zero : slot[label]; };
+    for (int k = 0; k <= steps; ++k) {
+      const Pair& pr = sched[is][k];
+      lv[k] = {slot_of(pr.a), slot_of(pr.b), pr.f, b0, b1, 0.f, 0};
+      const int it = nt - 3 - k;
+      if (k < steps && it >= ntNeg && nri > 0) {
+        const float fr = (it - ntNeg + 1.) / ratio;
+        const int i1 = (int)fr;
+        if ((it - ntNeg + 2) % ratio == 0) {  // row i1 enters, the older row leaves
+          b1 = i1;
+          std::swap(b0, b1);
+        }
+        lv[k].r0 = b0;
+        lv[k].r1 = b1;
+        lv[k].fi = fr - i1;
+        lv[k].inject = 1;
+      }
+    }
+    auto up = [&](void* d, const void* h, size_t bytes) {
+      return cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s);
+    };
+    VTI_CUDA(ctx, up(d_cells, cells.data(), cells.size() * sizeof(int)));
+    VTI_CUDA(ctx, up(d_row, row.data(), nt * sizeof(int)));
+    VTI_CUDA(ctx, up(d_keep, keep.data(), nt * sizeof(int)));
+    VTI_CUDA(ctx, up(d_amp, amp.data(), nt * sizeof(float)));
+    VTI_CUDA(ctx, up(d_src, &src, sizeof(int)));
+    VTI_CUDA(ctx, up(d_nri, &nri, sizeof(int)));
+    VTI_CUDA(ctx, up(d_lv, lv.data(), lv.size() * sizeof(tile2d::BackLevel)));
+    int st = tile2d::launch_map(ctx, L, d_cells, nri, d_map);
+    if (st != VTI_OK) return st;
+    VTI_CUDA(ctx, cudaMemsetAsync(rec, 0, (size_t)nnt_data * std::max(nri, 1) * sizeof(float), s));
+    // ---- forward
+    VTI_CUDA(ctx, cudaMemsetAsync(waves, 0, tile2d::kWaveArrays * L.n * sizeof(float), s));
+    st = tile2d::launch_point(ctx, waves, waves + L.n, src, dt2 * wavelet[0]);  // no taper
+    if (st != VTI_OK) return st;
+    float *in = waves, *other = waves + 4 * L.n;
+    for (int it = 2; it < nt; it += L.T) {
+      f.lev0 = it;
+      f.nlev = std::min(L.T, nt - it);
+      f.in = in;
+      f.out = other;
+      st = tile2d::launch_forward(ctx, f);
+      if (st != VTI_OK) return st;
+      std::swap(in, other);
+    }
+    if (keep[nt - 1] >= 0) {
+      // the last level has no next step to carry its D: one more level, traces
+      // off, whose result is not used (row[] and amp[] hold nt entries)
+      tile2d::Forward last = f;
+      last.lev0 = nt;
+      last.nlev = 1;
+      last.in = in;
+      last.out = other;
+      last.rec_row = nullptr;
+      last.amp = d_amp - 1;  // amp of level nt: any value
+      st = tile2d::launch_forward(ctx, last);
+      if (st != VTI_OK) return st;
+    }
+    if (nri > 0) {
+      // residual and FP64 misfit (objFuncGradient_f.cu:214-219)
+      VTI_CUDA(ctx, cudaMemcpy2DAsync(obs, nri * sizeof(float), data + ir0,
+                                      (size_t)nr * sizeof(float), nri * sizeof(float), nnt_data,
+                                      cudaMemcpyHostToDevice, s));
+      st = launch_residual(ctx, rec, obs, live, nri, nnt_data, d_acc);
+      if (st != VTI_OK) return st;
+    }
+    // ---- backward
+    VTI_CUDA(ctx, cudaMemsetAsync(waves, 0, tile2d::kWaveArrays * L.n * sizeof(float), s));
+    in = waves;
+    other = waves + 4 * L.n;
+    st = tile2d::launch_inject(ctx, L, in, in + L.n, rec + (size_t)(nnt_data - 1) * nri, d_cells,
+                               nri, nullptr, dt2, 0, 0);
+    if (st != VTI_OK) return st;
+    tile2d::Backward b{};
+    b.L = L;
+    b.m = f.m;
+    b.exact = 1;
+    b.kept = kept;
+    b.g = grad;
+    b.rmap = nri > 0 ? d_map : nullptr;
+    b.rows = rec;
+    b.row_stride = nri;
+    for (int k = 0; k < steps; k += L.T) {
+      b.nlev = std::min(L.T, steps - k);
+      b.image_last = k + b.nlev == steps;
+      b.lv = d_lv + k;
+      b.in = in;
+      b.out = other;
+      st = tile2d::launch_backward(ctx, b);
+      if (st != VTI_OK) return st;
+      std::swap(in, other);
+    }
+    VTI_CUDA(ctx, cudaStreamSynchronize(s));  // per-shot host vectors
+  }
+  float* outs[3] = {gc11, gc13, gc33};
+  for (int k = 0; k < 3; ++k) {
+    const int st = tile2d::launch_unpad(ctx, L, grad + k * L.n, flat);
+    if (st != VTI_OK) return st;
+    VTI_CUDA(ctx, cudaMemcpyAsync(outs[k], flat, nnxz * sizeof(float), cudaMemcpyDeviceToHost, s));
+  }
+  double acc = 0;
+  VTI_CUDA(ctx, cudaMemcpyAsync(&acc, d_acc, sizeof(double), cudaMemcpyDeviceToHost, s));
+  VTI_CUDA(ctx, cudaStreamSynchronize(s));
+  if (misfit) *misfit = 0.5 * acc;
+  return VTI_OK;
+}
+
 int run_grad2d(vti_ctx* ctx, const vti2d_geom* g, float* gc11, float* gc13, float* gc33,
                const float* data, const float* c11, const float* c13, const float* c33,
                const float* dc11, const float* dc13, const float* dc33, const float* wavelet,
@@ -397,6 +617,11 @@ int run_grad2d(vti_ctx* ctx, const vti2d_geom* g, float* gc11, float* gc13, floa
       if (p.b >= 0 && !slot.count(p.b)) slot[p.b] = (int)slot.size();
     }
   const int nslot = (int)slot.size();
+  if (!born) {
+    const int tst = grad2d_tiles(ctx, g, gc11, gc13, gc33, data, c11, c13, c33, wavelet, sloc, ns,
+                                 rloc, nr, taper, misfit, sched, slot, ratio, ntNeg, nnt_data);
+    if (tst != VTI_ERR_UNSUPPORTED) return tst;
+  }
   // device memory: model 3 (+3 dc) + taper + 4 fields (+4 Born) + 3 gradients
   // + 2 D buffers per checkpoint
   const size_t nfield = 3 + (born ? 3 : 0) + 1 + 4 + (born ? 4 : 0) + 3 + 2 + (born ? 2 : 0);

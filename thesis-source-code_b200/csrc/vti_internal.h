@@ -72,7 +72,7 @@ struct vti_ctx {
   std::vector<cudaEvent_t> event_pool;
   // 2D traces of grids that fit one thread-block cluster run shared-memory resident
   bool resident2d = true;
-  // device scratch of the 2D forward forms, kept between calls
+  // device scratch of the 2D forms, kept between calls
   float* scratch2d = nullptr;
   size_t scratch2d_bytes = 0;
   // staging block of host transfers of pitched volumes, kept between calls
@@ -159,6 +159,13 @@ int cuda_check(vti_ctx* ctx, cudaError_t e, const char* what);
     cudaError_t e_ = cudaGetLastError();                                     \
     if (e_ != cudaSuccess) return ::vti::cuda_check(ctx, e_, what);          \
   } while (0)
+
+// The context's 2D scratch of at least `bytes` bytes (kept between calls, freed
+// with the context). Gradients and migrations use it up to kScratch2dKeep, which a
+// 461 x 261 gradient of 1800 levels reaches, and allocate per call beyond: one of
+// 590 MB costs 1 to 4 ms of a 6 ms call in cudaMalloc and cudaFree.
+constexpr size_t kScratch2dKeep = (size_t)1 << 30;
+int scratch2d(vti_ctx* ctx, size_t bytes, float** out);
 
 int vol_alloc(vti_ctx* ctx, const Dims3& d, Vol* v);
 void vol_free(Vol* v);

@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "vti_internal.h"
+#include "vti_tile2d.h"
 
 namespace vti {
 namespace {
@@ -146,6 +147,196 @@ using namespace vti;
 
 namespace {
 
+// rtm_f through the tiled kernels (vti_tile2d.cu): receivers of a shot, with the
+// row below them, in the update region and on different cells. The same levels,
+// slices and injections as rtm2d_impl, which has checked the arguments.
+// VTI_ERR_UNSUPPORTED: not eligible, nothing was computed.
+int rtm2d_tiles(vti_ctx* ctx, const vti2d_geom* g, float* image, const float* data,
+                const float* c11, const float* c13, const float* c33, const float* wavelet,
+                const int* sloc, int ns, const int* rloc, int nr, const float* taper) {
+  const int nnx = g->nx + 2 * g->npad, nnz = g->nz + 2 * g->npad, nt = g->nt;
+  const size_t nnxz = (size_t)nnx * nnz;
+  if (!ctx->resident2d || nnxz > (1u << 30)) return VTI_ERR_UNSUPPORTED;
+  for (int is = 0; is < ns; ++is)
+    if (!tile2d::receivers_fit(nnx, nnz, rloc + 2 * sloc[4 * is + 3], sloc[4 * is + 2], true))
+      return VTI_ERR_UNSUPPORTED;
+  const float dt = g->dt, dt2 = dt * dt;
+  const int ratio = (int)(g->rate / dt + 0.5f);
+  const int ntNeg = (int)std::round(std::fabs(g->ot) / dt);
+  const int nnt = (nt - 1) / ratio + 1, nnt_data = (nt - ntNeg - 1) / ratio + 1;
+  const tile2d::Layout L = tile2d::make_layout(ctx, nnx, nnz, 1, true);
+  VTI_CUDA(ctx, cudaSetDevice(ctx->device));
+  float *flat, *model, *waves, *img, *slices, *ddata, *d_amp;
+  int *d_map, *d_keep, *d_src, *d_cells;
+  tile2d::BackLevel* d_lv;
+  struct Block {  // larger than the context keeps
+    float* p = nullptr;
+    ~Block() {
+      if (p) cudaFree(p);
+    }
+  } own;
+  float* block = nullptr;
+  const size_t n_data = (size_t)std::max(nnt_data, 0) * nr;
+  for (int pass = 0; pass < 2; ++pass) {
+    tile2d::Carve c{reinterpret_cast<char*>(block)};
+    flat = c.take<float>(nnxz);
+    model = c.take<float>(4 * L.n);
+    waves = c.take<float>(tile2d::kWaveArrays * L.n);
+    img = c.take<float>(L.n);
+    slices = c.take<float>(((size_t)nnt + 1) * L.n);  // one past the last slice reads zeros
+    ddata = c.take<float>(std::max<size_t>(n_data, 1));
+    d_map = c.take<int>(L.n);
+    d_amp = c.take<float>(nt);
+    d_keep = c.take<int>(nt);
+    d_src = c.take<int>(1);
+    d_cells = c.take<int>(std::max(nr, 1));
+    d_lv = c.take<tile2d::BackLevel>(nt);
+    if (pass) break;
+    if (c.used <= kScratch2dKeep) {
+      const int st = scratch2d(ctx, c.used, &block);
+      if (st != VTI_OK) return st;
+    } else {
+      VTI_CUDA(ctx, cudaMalloc((void**)&own.p, c.used));
+      block = own.p;
+    }
+  }
+  cudaStream_t s = ctx->stream;
+  VTI_CUDA(ctx, cudaMemsetAsync(model, 0, 4 * L.n * sizeof(float), s));
+  const float* host[4] = {c11, c13, c33, taper};
+  int st = VTI_OK;
+  for (int k = 0; k < 4 && st == VTI_OK; ++k) {
+    VTI_CUDA(ctx, cudaMemcpyAsync(flat, host[k], nnxz * sizeof(float), cudaMemcpyHostToDevice, s));
+    st = tile2d::launch_pad(ctx, L, flat, model + k * L.n, true);
+  }
+  if (st != VTI_OK) return st;
+  if (n_data)
+    VTI_CUDA(ctx, cudaMemcpyAsync(ddata, data, n_data * sizeof(float), cudaMemcpyHostToDevice, s));
+  // image and every slice start at zero (rtm_f.cu:24,55)
+  VTI_CUDA(ctx, cudaMemsetAsync(img, 0, L.n * sizeof(float), s));
+  VTI_CUDA(ctx, cudaMemsetAsync(slices, 0, ((size_t)nnt + 1) * L.n * sizeof(float), s));
+  tile2d::Forward f{};
+  f.L = L;
+  f.m = {model, model + L.n, model + 2 * L.n, model + 3 * L.n, 1.f / (g->dx * g->dx),
+         1.f / (g->dz * g->dz), dt2};
+  f.shots = 1;
+  f.src = d_src;
+  f.amp = d_amp;
+  f.dipole = 1;
+  f.keep_mode = tile2d::kKeepSlice;
+  f.keep = d_keep;
+  f.kept = slices;
+  std::vector<int> keep(nt, -1);
+  std::vector<float> amp(nt, 0.f);
+  for (int it = 2; it < nt; ++it) {
+    if (it % ratio == 0) keep[it] = it / ratio;
+    amp[it] = dt2 * wavelet[it - 1];
+  }
+  // backward levels: slices each level is imaged with, rows each injection reads
+  const int steps = nt - 2;
+  std::vector<tile2d::BackLevel> lv(steps + 1);
+  {
+    float fs = (nt - 2.) / ratio;
+    int s0 = (int)fs, s1 = std::min(s0 + 1, nnt);
+    fs -= s0;
+    int d0 = nnt_data - 1, d1 = -1;
+    for (int k = 0; k <= steps; ++k) {
+      const int it = nt - 3 - k;
+      lv[k] = {s0, s1, fs, d0, d1, 0.f, 0};
+      if (k == steps) break;
+      if (it >= ntNeg) {
+        float fd = (it - ntNeg + 1.) / ratio;
+        const int i1 = (int)fd;
+        if ((it - ntNeg + 2) % ratio == 0) {
+          d1 = i1;
+          std::swap(d0, d1);
+        }
+        lv[k].r0 = d0;
+        lv[k].r1 = d1;
+        lv[k].fi = fd - i1;
+        lv[k].inject = 1;
+      }
+      fs = (float)it / ratio;
+      const int i1 = (int)fs;
+      if ((it + 1) % ratio == 0) {
+        s1 = i1;
+        std::swap(s0, s1);
+      }
+      fs -= i1;
+    }
+  }
+  auto up = [&](void* d, const void* h, size_t bytes) {
+    return cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s);
+  };
+  VTI_CUDA(ctx, up(d_keep, keep.data(), nt * sizeof(int)));
+  VTI_CUDA(ctx, up(d_amp, amp.data(), nt * sizeof(float)));
+  VTI_CUDA(ctx, up(d_lv, lv.data(), lv.size() * sizeof(tile2d::BackLevel)));
+  for (int is = 0; is < ns; ++is) {
+    const int* sh = sloc + 4 * is;
+    const int nri = sh[2], ir0 = sh[3], src = L.at(sh[0], sh[1]);
+    const size_t sxz = sh[0] + (size_t)sh[1] * nnx;
+    std::vector<int> cells(std::max(nri, 1));
+    for (int ir = 0; ir < nri; ++ir)
+      cells[ir] = L.at(rloc[2 * (ir0 + ir)], rloc[2 * (ir0 + ir) + 1]);
+    VTI_CUDA(ctx, up(d_cells, cells.data(), cells.size() * sizeof(int)));
+    VTI_CUDA(ctx, up(d_src, &src, sizeof(int)));
+    st = tile2d::launch_map(ctx, L, d_cells, nri, d_map);
+    if (st != VTI_OK) return st;
+    // level 1 (rtm_f.cu:113-120): the dipole, then the taper; with ratio 1 its slice
+    // 0.5(p+q) holds the same two values
+    VTI_CUDA(ctx, cudaMemsetAsync(waves, 0, tile2d::kWaveArrays * L.n * sizeof(float), s));
+    const float a0 = dt2 * wavelet[0];
+    const float v[2] = {taper[sxz] * a0, -(taper[sxz + nnx] * a0)};
+    if (ratio == 1) VTI_CUDA(ctx, cudaMemsetAsync(slices + L.n, 0, L.n * sizeof(float), s));
+    for (int e = 0; e < 2; ++e) {
+      st = tile2d::launch_point(ctx, waves, waves + L.n, src + e * L.W, v[e]);
+      if (st == VTI_OK && ratio == 1)
+        st = tile2d::launch_point(ctx, slices + L.n, slices + L.n, src + e * L.W, v[e]);
+      if (st != VTI_OK) return st;
+    }
+    float *in = waves, *other = waves + 4 * L.n;
+    for (int it = 2; it < nt; it += L.T) {
+      f.lev0 = it;
+      f.nlev = std::min(L.T, nt - it);
+      f.in = in;
+      f.out = other;
+      st = tile2d::launch_forward(ctx, f);
+      if (st != VTI_OK) return st;
+      std::swap(in, other);
+    }
+    // receiver pass (rtm_f.cu:152-225)
+    VTI_CUDA(ctx, cudaMemsetAsync(waves, 0, tile2d::kWaveArrays * L.n * sizeof(float), s));
+    in = waves;
+    other = waves + 4 * L.n;
+    st = tile2d::launch_inject(ctx, L, in, in + L.n, ddata + ir0 + (size_t)(nnt_data - 1) * nr,
+                               d_cells, nri, f.m.taper, dt2, 1, 1);
+    if (st != VTI_OK) return st;
+    tile2d::Backward b{};
+    b.L = L;
+    b.m = f.m;
+    b.kept = slices;
+    b.g = img;
+    b.rmap = nri > 0 ? d_map : nullptr;
+    b.rows = ddata + ir0;
+    b.row_stride = nr;
+    for (int k = 0; k < steps; k += L.T) {
+      b.nlev = std::min(L.T, steps - k);
+      b.image_last = k + b.nlev == steps;
+      b.lv = d_lv + k;
+      b.in = in;
+      b.out = other;
+      st = tile2d::launch_backward(ctx, b);
+      if (st != VTI_OK) return st;
+      std::swap(in, other);
+    }
+    VTI_CUDA(ctx, cudaStreamSynchronize(s));  // per-shot host values
+  }
+  st = tile2d::launch_unpad(ctx, L, img, flat);
+  if (st != VTI_OK) return st;
+  VTI_CUDA(ctx, cudaMemcpyAsync(image, flat, nnxz * sizeof(float), cudaMemcpyDeviceToHost, s));
+  VTI_CUDA(ctx, cudaStreamSynchronize(s));
+  return VTI_OK;
+}
+
 // rtm_f (nhx < 0) and odcig_f (nhx >= 0, lib/vti-fwi-2d/odcig_f.cu:12-232):
 // the same passes; odcig_f images with subsurface x offsets |h| <= nhx and its
 // source pass injects w[it-1] without the dt2 factor after level 1
@@ -180,6 +371,11 @@ int rtm2d_impl(vti_ctx* ctx, const vti2d_geom* g, int nhx, float* image, const f
       if (x < 0 || x >= nnx || z < 0 || z + 1 >= nnz)
         return fail(ctx, VTI_ERR_ARG, "2D receiver (and the point below it) outside the grid");
     }
+  }
+  if (nhx < 0 && nnt_data >= 1) {
+    const int tst = rtm2d_tiles(ctx, g, image, data, c11, c13, c33, wavelet, sloc, ns, rloc, nr,
+                                taper);
+    if (tst != VTI_ERR_UNSUPPORTED) return tst;
   }
   VTI_CUDA(ctx, cudaSetDevice(ctx->device));
   cudaStream_t sm = ctx->stream;
