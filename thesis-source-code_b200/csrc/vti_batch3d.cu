@@ -472,12 +472,14 @@ int backward_loop(vti3d_batch* b) {
   return VTI_OK;
 }
 
-// Ratio of the side-by-side step kernels' HBM bandwidth to the single-grid
-// kernels' (measured on windows of 160..400 x 160..400 x 200 cells: 0.64 and
-// 0.81 of the copy bandwidth for the backward step), and the gap between two
-// single-grid launches in CTA-slot plane-steps (about 3 us; one plane-step
-// of a 32 x 16 column is about 2 us).
-constexpr double kSideBySideRel = 0.79;
+// Speed of the side-by-side step kernels relative to the single-grid kernels
+// on windows that fill the GPU (whole gradients with the alternating march, six
+// and 16 windows of 160..400 x 160..400 x 200 cells: 0.90 to 0.94; it was 0.79 when
+// both marched one way), and the gap between two single-grid launches in CTA-slot
+// plane-steps (about 3 us; one plane-step of a 32 x 16 column is about 2 us).
+// Windows whose schedule keeps the SMs less busy lose side by side nothing or
+// gain up to 4 % (160x160x150, 224x224x100).
+constexpr double kSideBySideRel = 0.9;
 constexpr long long kLaunchGap = 2;
 
 // The schedule of the next gradient: the one set; under auto the one

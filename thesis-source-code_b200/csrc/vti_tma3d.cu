@@ -792,8 +792,15 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 // Segment length: the smallest modelled time, counted in plane-steps of one
 // CTA, waves * (seg + restart), where a wave is one item per resident slot
 // and a restart (8 queue planes read with plain loads, pipeline refill) costs
-// about kRestart plane-steps.
-constexpr long long kRestart = 4;
+// about kRestart plane-steps. Segments of fewer than 8 planes (down to 4) only
+// while all items are resident at once: there they fill slots that would idle,
+// with more waves they only add restarts.
+// Measured with the alternating march (nt 300..514), restart 4 -> 1: gradient
+// 300x200x90 50.3 -> 46.8 ms, 251x203x150 89.4 -> 87.9, 400x400x200 and
+// 128^3..208x192x128 unchanged; short segments: 110x97x83 one-call 22.7 -> 20.4 ms,
+// 112x112x96 12.2 -> 11.7 ms, allowed everywhere 160x160x112 25.0 -> 25.5 ms.
+constexpr long long kRestart = 1;
+constexpr int kSegPlanes = 8, kSegPlanesOneWave = 4;
 
 Sched make_sched(vti_ctx* ctx, const Dims3& d, int ctas_per_sm) {
   Sched s;
@@ -805,11 +812,12 @@ Sched make_sched(vti_ctx* ctx, const Dims3& d, int ctas_per_sm) {
   long long best = -1;
   for (int nseg = 1; nseg <= d.nz; ++nseg) {
     const int seg = (d.nz + nseg - 1) / nseg;
-    if (nseg > 1 && seg < 8) break;  // at least 8 planes per queue start
+    if (nseg > 1 && seg < kSegPlanesOneWave) break;
     if (nseg > 1 && seg == (d.nz + nseg - 2) / (nseg - 1)) continue;  // same seg
     const long long items = cols * ((d.nz + seg - 1) / seg);
     if (items > (1LL << 30)) break;
     const long long waves = (items + slots - 1) / slots;
+    if (nseg > 1 && seg < kSegPlanes && waves > 1) continue;
     const long long cost = waves * (seg + kRestart);
     if (best < 0 || cost < best) {
       best = cost;
