@@ -63,11 +63,10 @@ struct BornMaps {
   CUtensorMap ax, bx, az, bz, apx, apz, bpx, bpz, c11, c13, c33, d11, d13, d33;
 };
 // Born step stage: two halo tiles (x fields) and 12 plain tiles (the two z
-// fields 4 planes below, the four previous-level tiles, the model and the
+// fields 4 planes ahead, the four previous-level tiles, the model and the
 // perturbation), three stages. Reading the model and the perturbation with
-// read-only loads instead (as the adjoint does) measured 4 % slower here:
-// the kernel already spills at 96 registers and the six pairs held across
-// the stage wait add to it.
+// read-only loads instead (as the adjoint does) measured 4 % slower when the
+// scalar form of this kernel spilled at 96 registers.
 constexpr int GB_STAGES = 3;
 constexpr int G_OFF_P = 2 * HALO_BYTES;
 constexpr int GB_STAGE_BYTES = G_OFF_P + 12 * PLAIN_BYTES;  // 32256
@@ -96,33 +95,75 @@ __device__ __forceinline__ void ldg3(const float* p0, const float* p1, const flo
 
 // Loads of one item: two halo tiles (x fields) and kNumPlain plain tiles per
 // plane, into a ring of kStages stages of kStageBytes.
-template <typename Maps, int kNumPlain, int kStages, int kStageBytes>
+template <typename Maps, int kNumPlain, int kStages, int kStageBytes, int kDir>
 __device__ __forceinline__ bool produce14(const Sched& sc, const Maps& m, int* status, int li,
                                           unsigned char* smem, uint64_t* full, uint64_t* empty,
-                                          long long& k) {
+                                          RingPos<kStages>& k) {
   static_assert(sizeof(Maps) == (2 + kNumPlain) * sizeof(CUtensorMap), "map layout");
   static_assert(2 * HALO_BYTES + kNumPlain * PLAIN_BYTES <= kStageBytes, "stage size");
   const CUtensorMap* maps = reinterpret_cast<const CUtensorMap*>(&m);
   int bx, by, z0, z1;
   item(sc, li, bx, by, z0, z1);
   const int x0 = bx * TX, y0 = kHalo + by * TY;
-  for (int z = z0; z < z1; ++z, ++k) {
-    const int s = (int)(k % kStages);
-    if (k >= kStages && !mbar_wait(&empty[s], (uint32_t)(((k / kStages) & 1) ^ 1), status))
-      return false;
+  for (int n = 0; n < z1 - z0; ++n, k.advance()) {
+    const int z = kDir > 0 ? z0 + n : z1 - 1 - n;
+    const int s = k.s;
+    if (!mbar_wait(&empty[s], k.ph ^ 1u, status)) return false;
     const int zp = z + kZPad;
     unsigned char* st = smem + s * kStageBytes;
     mbar_arrive_expect_tx(&full[s], 2 * HALO_BYTES + kNumPlain * PLAIN_BYTES);
     tma_load(st, &maps[0], &full[s], x0 - kHalo, y0 - kHalo, zp);
     tma_load(st + HALO_BYTES, &maps[1], &full[s], x0 - kHalo, y0 - kHalo, zp);
-    // plain tiles 0, 1: the z fields 4 planes below (register queues)
-    tma_load(st + G_OFF_P, &maps[2], &full[s], x0, y0, zp + kHalo);
-    tma_load(st + G_OFF_P + PLAIN_BYTES, &maps[3], &full[s], x0, y0, zp + kHalo);
+    // plain tiles 0, 1: the z fields 4 planes ahead (register queues)
+    tma_load(st + G_OFF_P, &maps[2], &full[s], x0, y0, zp + kDir * kHalo);
+    tma_load(st + G_OFF_P + PLAIN_BYTES, &maps[3], &full[s], x0, y0, zp + kDir * kHalo);
 #pragma unroll
     for (int j = 2; j < kNumPlain; ++j)
       tma_load(st + G_OFF_P + j * PLAIN_BYTES, &maps[2 + j], &full[s], x0, y0, zp);
   }
   return true;
+}
+
+// L_xy (forward-form scaled) of the x pair at h, the centre of a halo tile, as
+// packed FP32 pairs (each lane rounded as the scalar operation); *c its values.
+__device__ __forceinline__ float2 lxy_2(const float* h, float sx, float sy, float2* c) {
+  float r[10];
+#pragma unroll
+  for (int j = 0; j < 5; ++j) {
+    const float2 t = ld2(h - 4 + 2 * j);
+    r[2 * j] = t.x;
+    r[2 * j + 1] = t.y;
+  }
+  *c = make_float2(r[4], r[5]);
+  const float2 lyy = lap9_2(*c, ld2(h - HX), ld2(h + HX), ld2(h - 2 * HX), ld2(h + 2 * HX),
+                            ld2(h - 3 * HX), ld2(h + 3 * HX), ld2(h - 4 * HX), ld2(h + 4 * HX));
+  float2 lxx;
+  lxx.x = lap9(r[4], r[3], r[5], r[2], r[6], r[1], r[7], r[0], r[8]);
+  lxx.y = lap9(r[5], r[4], r[6], r[3], r[7], r[2], r[8], r[1], r[9]);
+  return fma2(lyy, splat(sy), mul2(lxx, splat(sx)));
+}
+__device__ __forceinline__ float2 lz_2(const float2 (&q)[9], float sz) {
+  return mul2(lap9_2(q[4], q[3], q[5], q[2], q[6], q[1], q[7], q[0], q[8]), splat(sz));
+}
+// Queue start of the march (one shift before the first plane, see queue_shift).
+template <int kDir>
+__device__ __forceinline__ void queue_start(float2 (&q)[9], const float* f, const Dims3& d, int off,
+                                            int z0, int z1, bool any) {
+  q[kDir > 0 ? 0 : 8] = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int kk = kDir > 0 ? 1 : 0; kk < (kDir > 0 ? 9 : 8); ++kk) {
+    const int zz = kDir > 0 ? z0 - 5 + kk : z1 - 4 + kk;
+    q[kk] = any ? __ldg(reinterpret_cast<const float2*>(f + (long long)zz * d.plane + off))
+                : make_float2(0.f, 0.f);
+  }
+}
+__device__ __forceinline__ void store_pair(float* p, float2 v, bool v0, bool v1) {
+  if (v0 && v1) {
+    *reinterpret_cast<float2*>(p) = v;
+  } else {
+    if (v0) p[0] = v.x;
+    if (v1) p[1] = v.y;
+  }
 }
 
 struct Stencil2 {  // the x-row, y-column and z-queue stencil of one x pair
@@ -181,18 +222,19 @@ __device__ __forceinline__ void queue_push(float (&q)[2][9], float2 v) {
   q[1][8] = v.y;
 }
 
+template <int kDir>
 __global__ void __launch_bounds__(NTHREADS, 2)
     k_born3d_tma(const __grid_constant__ BornMaps m, const __grid_constant__ BornArgs a) {
   extern __shared__ unsigned char smem_raw[];
   uint64_t *full, *empty;
   unsigned char* smem = ring_init<GB_STAGES, GB_STAGE_BYTES>(smem_raw, full, empty);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  long long k = 0;
+  RingPos<GB_STAGES> k;
   if (warp == NCW) {
     if (lane == 0)
-      for (int it = blockIdx.x; it < a.sc.items; it += gridDim.x)
-        if (!produce14<BornMaps, 12, GB_STAGES, GB_STAGE_BYTES>(a.sc, m, a.status, it, smem,
-                                                               full, empty, k))
+      for (int n = blockIdx.x; n < a.sc.items; n += gridDim.x)
+        if (!produce14<BornMaps, 12, GB_STAGES, GB_STAGE_BYTES, kDir>(
+                a.sc, m, a.status, march_item<kDir>(n, a.sc.items), smem, full, empty, k))
           break;
     return;
   }
@@ -200,79 +242,74 @@ __global__ void __launch_bounds__(NTHREADS, 2)
   const int xo = 2 * (lane & 15);
   const int sr = (ry + kHalo) * HX + xo + kHalo;
   const int pi = ry * TX + xo;
-  for (int it = blockIdx.x; it < a.sc.items; it += gridDim.x) {
+  for (int n = blockIdx.x; n < a.sc.items; n += gridDim.x) {
     int bx, by, z0, z1;
-    item(a.sc, it, bx, by, z0, z1);
+    item(a.sc, march_item<kDir>(n, a.sc.items), bx, by, z0, z1);
     const int x = bx * TX + xo;
     const int y = kHalo + by * TY + ry;
     const bool vy = y < a.d.ny - kHalo;
     const bool v0 = vy && x >= kHalo && x < a.d.nx - kHalo;
     const bool v1 = vy && x + 1 >= kHalo && x + 1 < a.d.nx - kHalo;
     const int off = y * a.d.pitch + x;
-    float aq[2][9], bq[2][9], dxy[2];
-    queue_init(aq, a.az, a.d, off, z0, v0 || v1);
-    queue_init(bq, a.bz, a.d, off, z0, v0 || v1);
-    dxy[0] = v0 ? a.dampx[x] * a.dampy[y] : 1.f;
-    dxy[1] = v1 ? a.dampx[x + 1] * a.dampy[y] : 1.f;
+    const int src_e = (y == a.src.y && a.src.x >= 0) ? a.src.x - x : -1;
+    float2 aq[9], bq[9];
+    queue_start<kDir>(aq, a.az, a.d, off, z0, z1, v0 || v1);
+    queue_start<kDir>(bq, a.bz, a.d, off, z0, z1, v0 || v1);
+    const float2 dxy = make_float2(v0 ? a.dampx[x] * a.dampy[y] : 1.f,
+                                   v1 ? a.dampx[x + 1] * a.dampy[y] : 1.f);
     bool ok = true;
-    for (int z = z0; z < z1; ++z, ++k) {
-      const float dz = a.dampz[z];
-      const int s = (int)(k % GB_STAGES);
-      if (!mbar_wait(&full[s], (uint32_t)((k / GB_STAGES) & 1), a.status)) {
+    const int zend = kDir > 0 ? z1 : z0 - 1;
+    for (int z = kDir > 0 ? z0 : z1 - 1; z != zend; z += kDir, k.advance()) {
+      const float2 dd = mul2(dxy, splat(__ldg(a.dampz + z)));
+      const int s = k.s;
+      if (!mbar_wait(&full[s], k.ph, a.status)) {
         ok = false;
         break;
       }
       const unsigned char* st = smem + s * GB_STAGE_BYTES;
       const float* pl = (const float*)(st + G_OFF_P) + pi;
       constexpr int T = TX * TY;
-      queue_push(aq, ld2(pl));
-      queue_push(bq, ld2(pl + T));
-      Stencil2 sa, sb;
-      sa.load((const float*)st + sr);
-      sb.load((const float*)(st + HALO_BYTES) + sr);
-      const float2 apx = ld2(pl + 2 * T), apz = ld2(pl + 3 * T);
-      const float2 bpx = ld2(pl + 4 * T), bpz = ld2(pl + 5 * T);
+      queue_shift<kDir>(aq, ld2(pl));
+      queue_shift<kDir>(bq, ld2(pl + T));
+      // one field's stencil after the other, the model last (shorter live ranges:
+      // no spills at the 96 registers of two CTAs per SM)
+      float2 ac, bc;
+      const float2 lxy = lxy_2((const float*)st + sr, a.sx, a.sy, &ac);
+      const float2 lz = lz_2(aq, a.sz);
+      const float2 blxy = lxy_2((const float*)(st + HALO_BYTES) + sr, a.sx, a.sy, &bc);
+      const float2 blz = lz_2(bq, a.sz);
       const float2 c11 = ld2(pl + 6 * T), c13 = ld2(pl + 7 * T), c33 = ld2(pl + 8 * T);
       const float2 d11 = ld2(pl + 9 * T), d13 = ld2(pl + 10 * T), d33 = ld2(pl + 11 * T);
+      const float2 two = splat(2.f), npc = sub2(splat(1.f), mul2(two, dd));
+      // scattering source dC L a_{t-1} of the Born field
+      const float2 sx_ = fma2(d11, lxy, mul2(d13, lz));
+      const float2 sz_ = fma2(d13, lxy, mul2(d33, lz));
+      // background: the exact forward step (same expression as k_fwd3d_tma),
+      // centred damping: - (2D - 1) prev
+      float2 anx = fma2(c11, lxy, fma2(c13, lz, mul2(two, ac)));
+      float2 anz = fma2(c13, lxy, fma2(c33, lz, mul2(two, aq[4])));
+      if (z == a.src.z) {
+        if (src_e == 0) {
+          anx.x += a.src.amp;
+          anz.x += a.src.amp;
+        }
+        if (src_e == 1) {
+          anx.y += a.src.amp;
+          anz.y += a.src.amp;
+        }
+      }
+      anx = fma2(dd, anx, mul2(npc, ld2(pl + 2 * T)));
+      anz = fma2(dd, anz, mul2(npc, ld2(pl + 3 * T)));
+      const float2 bx_ = add2(fma2(c11, blxy, fma2(c13, blz, mul2(two, bc))), sx_);
+      const float2 bz_ = add2(fma2(c13, blxy, fma2(c33, blz, mul2(two, bq[4]))), sz_);
+      const float2 bnx = fma2(dd, bx_, mul2(npc, ld2(pl + 4 * T)));
+      const float2 bnz = fma2(dd, bz_, mul2(npc, ld2(pl + 5 * T)));
       stage_release(&empty[s], lane);
-      float anx[2], anz[2], bnx[2], bnz[2];
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        auto pick = [e](float2 v) { return e ? v.y : v.x; };
-        const float dd = dxy[e] * dz;
-        const float a11 = pick(c11), a13 = pick(c13), a33 = pick(c33);
-        // background: the exact forward step (same expression as k_fwd3d_tma)
-        const float lxy = sa.lxy(e, a.sx, a.sy);
-        const float lz = lz_of(aq[e], a.sz);
-        const float pc = 2.f * dd - 1.f;  // centred damping: - (2D - 1) prev
-        anx[e] = fmaf(a11, lxy, fmaf(a13, lz, 2.f * sa.r[4 + e]));
-        anz[e] = fmaf(a13, lxy, fmaf(a33, lz, 2.f * aq[e][4]));
-        if (x + e == a.src.x && y == a.src.y && z == a.src.z) {
-          anx[e] += a.src.amp;
-          anz[e] += a.src.amp;
-        }
-        anx[e] = fmaf(dd, anx[e], -pc * pick(apx));
-        anz[e] = fmaf(dd, anz[e], -pc * pick(apz));
-        // Born field: same operator plus the scattering source dC L a_{t-1}
-        const float blxy = sb.lxy(e, a.sx, a.sy);
-        const float blz = lz_of(bq[e], a.sz);
-        const float sx_ = fmaf(pick(d11), lxy, pick(d13) * lz);
-        const float sz_ = fmaf(pick(d13), lxy, pick(d33) * lz);
-        bnx[e] = fmaf(dd, fmaf(a11, blxy, fmaf(a13, blz, 2.f * sb.r[4 + e])) + sx_,
-                      -pc * pick(bpx));
-        bnz[e] = fmaf(dd, fmaf(a13, blxy, fmaf(a33, blz, 2.f * bq[e][4])) + sz_,
-                      -pc * pick(bpz));
-      }
       const long long i = (long long)z * a.d.plane + off;
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        if (e ? v1 : v0) {
-          a.apx[i + e] = anx[e];
-          a.apz[i + e] = anz[e];
-          a.bpx[i + e] = bnx[e];
-          a.bpz[i + e] = bnz[e];
-        }
-      }
+      store_pair(a.apx + i, anx, v0, v1);
+      store_pair(a.apz + i, anz, v0, v1);
+      store_pair(a.bpx + i, bnx, v0, v1);
+      store_pair(a.bpz + i, bnz, v0, v1);
     }
     if (!ok) break;
   }
@@ -304,94 +341,95 @@ struct AdjMaps {
   CUtensorMap wx, ax, wz, az, m1x, m1z, mpx, mpz;
 };
 
+// The images of one launch (gradient, H dc, or both) side by side: item n is
+// item n / images of image n % images, so two CTAs that run together read the
+// same background and model planes, and the second finds them in L2 (20 of the
+// 84 bytes per point). Both Gauss-Newton kernels alternate the march direction
+// (queue_shift) and work on packed FP32 pairs. 200x180x120, nt 300, whole product
+// with both images: 108 -> 95.5 ms, bitwise the same sums.
+struct AdjLaunch {
+  AdjMaps m[2];
+  AdjArgs a[2];
+  int images;
+};
+
+template <int kDir>
 __global__ void __launch_bounds__(NTHREADS, 2)
-    k_adj3d_tma(const __grid_constant__ AdjMaps m, const __grid_constant__ AdjArgs a) {
+    k_adj3d_tma(const __grid_constant__ AdjLaunch L) {
   extern __shared__ unsigned char smem_raw[];
   uint64_t *full, *empty;
   unsigned char* smem = ring_init<G_STAGES, G_STAGE_BYTES>(smem_raw, full, empty);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  long long k = 0;
+  RingPos<G_STAGES> k;
+  const int items = L.a[0].sc.items * L.images;
   if (warp == NCW) {
     if (lane == 0)
-      for (int it = blockIdx.x; it < a.sc.items; it += gridDim.x)
-        if (!produce14<AdjMaps, 6, G_STAGES, G_STAGE_BYTES>(a.sc, m, a.status, it, smem, full,
-                                                            empty, k))
+      for (int n = blockIdx.x; n < items; n += gridDim.x) {
+        const int u = march_item<kDir>(n, items), im = u % L.images;
+        if (!produce14<AdjMaps, 6, G_STAGES, G_STAGE_BYTES, kDir>(
+                L.a[0].sc, L.m[im], L.a[0].status, u / L.images, smem, full, empty, k))
           break;
+      }
     return;
   }
   const int ry = warp * 2 + (lane >> 4);
   const int xo = 2 * (lane & 15);
   const int sr = (ry + kHalo) * HX + xo + kHalo;
   const int pi = ry * TX + xo;
-  for (int it = blockIdx.x; it < a.sc.items; it += gridDim.x) {
+  for (int n = blockIdx.x; n < items; n += gridDim.x) {
+    const int u = march_item<kDir>(n, items);
+    const AdjArgs& a = L.a[u % L.images];
     int bx, by, z0, z1;
-    item(a.sc, it, bx, by, z0, z1);
+    item(a.sc, u / L.images, bx, by, z0, z1);
     const int x = bx * TX + xo;
     const int y = kHalo + by * TY + ry;
     const bool vy = y < a.d.ny - kHalo;
     const bool v0 = vy && x >= kHalo && x < a.d.nx - kHalo;
     const bool v1 = vy && x + 1 >= kHalo && x + 1 < a.d.nx - kHalo;
     const int off = y * a.d.pitch + x;
-    float wq[2][9], aq[2][9], dxy[2];
-    queue_init(wq, a.wz, a.d, off, z0, v0 || v1);
-    queue_init(aq, a.az, a.d, off, z0, v0 || v1);
-    dxy[0] = v0 ? a.dampx[x] * a.dampy[y] : 1.f;
-    dxy[1] = v1 ? a.dampx[x + 1] * a.dampy[y] : 1.f;
+    float2 wq[9], aq[9];
+    queue_start<kDir>(wq, a.wz, a.d, off, z0, z1, v0 || v1);
+    queue_start<kDir>(aq, a.az, a.d, off, z0, z1, v0 || v1);
+    const float2 dxy = make_float2(v0 ? a.dampx[x] * a.dampy[y] : 1.f,
+                                   v1 ? a.dampx[x + 1] * a.dampy[y] : 1.f);
     bool ok = true;
     const bool any = v0 || v1;
-    for (int z = z0; z < z1; ++z, ++k) {
-      const float dz = a.dampz[z];
+    const int zend = kDir > 0 ? z1 : z0 - 1;
+    for (int z = kDir > 0 ? z0 : z1 - 1; z != zend; z += kDir, k.advance()) {
+      const float dz = __ldg(a.dampz + z);
       // issued before the stage wait; this thread alone writes its image cells
       float2 c11, c13, c33, g11o, g13o, g33o;
-      const long long gi = (long long)z * a.d.plane + off;
-      ldg3(a.c11, a.c13, a.c33, gi, any, c11, c13, c33);
-      ldg3(a.g11, a.g13, a.g33, gi, any, g11o, g13o, g33o);
-      const int s = (int)(k % G_STAGES);
-      if (!mbar_wait(&full[s], (uint32_t)((k / G_STAGES) & 1), a.status)) {
+      const long long i = (long long)z * a.d.plane + off;
+      ldg3(a.c11, a.c13, a.c33, i, any, c11, c13, c33);
+      ldg3(a.g11, a.g13, a.g33, i, any, g11o, g13o, g33o);
+      const int s = k.s;
+      if (!mbar_wait(&full[s], k.ph, a.status)) {
         ok = false;
         break;
       }
       const unsigned char* st = smem + s * G_STAGE_BYTES;
       const float* pl = (const float*)(st + G_OFF_P) + pi;
       constexpr int T = TX * TY;
-      queue_push(wq, ld2(pl));
-      queue_push(aq, ld2(pl + T));
-      Stencil2 sw, sa;
-      sw.load((const float*)st + sr);
-      sa.load((const float*)(st + HALO_BYTES) + sr);
+      queue_shift<kDir>(wq, ld2(pl));
+      queue_shift<kDir>(aq, ld2(pl + T));
+      float2 unused;
+      const float2 lxy = lxy_2((const float*)st + sr, a.sx, a.sy, &unused);  // L_xy w_x
+      const float2 axy = lxy_2((const float*)(st + HALO_BYTES) + sr, a.sx, a.sy, &unused);
       const float2 m1x = ld2(pl + 2 * T), m1z = ld2(pl + 3 * T);
       const float2 m2x = ld2(pl + 4 * T), m2z = ld2(pl + 5 * T);
       stage_release(&empty[s], lane);
-      float mx[2], mz[2], wx[2], wzv[2], g11[2], g13[2], g33[2];
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        auto pick = [e](float2 v) { return e ? v.y : v.x; };
-        const float dd = dxy[e] * dz;
-        const float lxy = sw.lxy(e, a.sx, a.sy);   // L_xy w_x
-        const float lz = lz_of(wq[e], a.sz);         // L_z w_z
-        mx[e] = fmaf(dd, 2.f * pick(m1x) + lxy, -(2.f * dd - 1.f) * pick(m2x));
-        mz[e] = fmaf(dd, 2.f * pick(m1z) + lz, -(2.f * dd - 1.f) * pick(m2z));
-        wx[e] = fmaf(pick(c11), mx[e], pick(c13) * mz[e]);
-        wzv[e] = fmaf(pick(c13), mx[e], pick(c33) * mz[e]);
-        const float axy = sa.lxy(e, a.sx, a.sy);   // L_xy a_{t-1,x}
-        const float az = lz_of(aq[e], a.sz);         // L_z a_{t-1,z}
-        g11[e] = fmaf(mx[e], axy, pick(g11o));
-        g13[e] = fmaf(mx[e], az, fmaf(mz[e], axy, pick(g13o)));
-        g33[e] = fmaf(mz[e], az, pick(g33o));
-      }
-      const long long i = (long long)z * a.d.plane + off;
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        if (e ? v1 : v0) {
-          a.mpx[i + e] = mx[e];
-          a.mpz[i + e] = mz[e];
-          a.wox[i + e] = wx[e];
-          a.woz[i + e] = wzv[e];
-          a.g11[i + e] = g11[e];
-          a.g13[i + e] = g13[e];
-          a.g33[i + e] = g33[e];
-        }
-      }
+      const float2 lz = lz_2(wq, a.sz), az = lz_2(aq, a.sz);  // L_z w_z, L_z a_{t-1,z}
+      const float2 two = splat(2.f), dd = mul2(dxy, splat(dz));
+      const float2 npc = sub2(splat(1.f), mul2(two, dd));
+      const float2 mx = fma2(dd, add2(mul2(two, m1x), lxy), mul2(npc, m2x));
+      const float2 mz = fma2(dd, add2(mul2(two, m1z), lz), mul2(npc, m2z));
+      store_pair(a.mpx + i, mx, v0, v1);
+      store_pair(a.mpz + i, mz, v0, v1);
+      store_pair(a.g11 + i, fma2(mx, axy, g11o), v0, v1);
+      store_pair(a.g13 + i, fma2(mx, az, fma2(mz, axy, g13o)), v0, v1);
+      store_pair(a.g33 + i, fma2(mz, az, g33o), v0, v1);
+      store_pair(a.wox + i, fma2(c11, mx, mul2(c13, mz)), v0, v1);
+      store_pair(a.woz + i, fma2(c13, mx, mul2(c33, mz)), v0, v1);
     }
     if (!ok) break;
   }
@@ -748,7 +786,7 @@ struct VolB {
 
 // once per device and kernel (atomic flags: first calls may come from
 // several host threads)
-std::atomic<bool> attr_born[64], attr_adj[64];
+std::atomic<bool> attr_born[2][64], attr_adj[2][64];
 
 int smem_attr(vti_ctx* ctx, const void* kern, std::atomic<bool>* done, int bytes = G_SMEM) {
   if (ctx->device < 64 && done[ctx->device].load(std::memory_order_acquire)) return VTI_OK;
@@ -816,9 +854,10 @@ struct GnState {
   }
 };
 
-int launch_born(GnState& S, int cur, const p3d::ShotGeom& sg, float amp) {
+int launch_born(GnState& S, int cur, const p3d::ShotGeom& sg, float amp, bool up) {
   vti_ctx* ctx = S.ctx;
-  VTI_TRY(smem_attr(ctx, (const void*)k_born3d_tma, attr_born, GB_SMEM));
+  const auto kern = up ? k_born3d_tma<-1> : k_born3d_tma<1>;
+  VTI_TRY(smem_attr(ctx, (const void*)kern, attr_born[up ? 1 : 0], GB_SMEM));
   const int nxt = 1 - cur;
   BornMaps m;
   m.ax = HM(S.a[cur][0].m);
@@ -851,54 +890,61 @@ int launch_born(GnState& S, int cur, const p3d::ShotGeom& sg, float amp) {
   x.status = ctx->d_status;
   {
     LaunchTimer tm(ctx, kTimedFwd3d);
-    k_born3d_tma<<<x.sc.grid, NTHREADS, GB_SMEM, ctx->stream>>>(m, x);
+    kern<<<x.sc.grid, NTHREADS, GB_SMEM, ctx->stream>>>(m, x);
   }
   VTI_LAUNCHED(ctx, "k_born3d_tma");
   return VTI_OK;
 }
 
-// Adjoint step of image `im` at level t: mu_{t+1} in mu[im][cur], mu_{t+2}
+// Adjoint step of the wanted images at level t: mu_{t+1} in mu[im][cur], mu_{t+2}
 // (overwritten by mu_t) in mu[im][1-cur], w_{t+1} in w[im][cur] (w_t into
-// w[im][1-cur]), a_{t-1} in segment slot `slot`.
-int launch_adj(GnState& S, int im, int cur, int slot) {
+// w[im][1-cur]), a_{t-1} in segment slot `slot`; up: the march's direction.
+int launch_adj(GnState& S, const bool (&want)[2], int cur, int slot, bool up) {
   vti_ctx* ctx = S.ctx;
-  VTI_TRY(smem_attr(ctx, (const void*)k_adj3d_tma, attr_adj));
+  const auto kern = up ? k_adj3d_tma<-1> : k_adj3d_tma<1>;
+  VTI_TRY(smem_attr(ctx, (const void*)kern, attr_adj[up ? 1 : 0], G_SMEM));
   const int nx_ = 1 - cur;
   const VolM* ax = &S.seg[2 * slot];
   const VolM* az = &S.seg[2 * slot + 1];
-  AdjMaps m;
-  m.wx = HM(S.w[im][cur][0].m);
-  m.ax = HM(ax->m);
-  m.wz = PM(S.w[im][cur][1].m);
-  m.az = PM(az->m);
-  m.m1x = PM(S.mu[im][cur][0].m);
-  m.m1z = PM(S.mu[im][cur][1].m);
-  m.mpx = PM(S.mu[im][nx_][0].m);
-  m.mpz = PM(S.mu[im][nx_][1].m);
   const float dt2 = S.g.dt * S.g.dt;
-  AdjArgs x{};
-  x.c11 = S.c[0].v.origin; x.c13 = S.c[1].v.origin; x.c33 = S.c[2].v.origin;
-  x.d = S.d;
-  x.sc = make_sched(ctx, S.d, 2);
-  x.wz = S.w[im][cur][1].v.origin;
-  x.az = az->v.origin;
-  x.mpx = S.mu[im][nx_][0].v.origin;
-  x.mpz = S.mu[im][nx_][1].v.origin;
-  x.wox = S.w[im][nx_][0].v.origin;
-  x.woz = S.w[im][nx_][1].v.origin;
-  x.g11 = S.img[im][0].v.origin;
-  x.g13 = S.img[im][1].v.origin;
-  x.g33 = S.img[im][2].v.origin;
-  x.dampx = S.damp;
-  x.dampy = S.damp + S.g.nx;
-  x.dampz = S.damp + S.g.nx + S.g.ny;
-  x.sx = dt2 / (S.g.dx * S.g.dx);
-  x.sy = dt2 / (S.g.dy * S.g.dy);
-  x.sz = dt2 / (S.g.dz * S.g.dz);
-  x.status = ctx->d_status;
+  AdjLaunch L{};
+  for (int im = 0; im < 2; ++im) {
+    if (!want[im]) continue;
+    AdjMaps& m = L.m[L.images];
+    m.wx = HM(S.w[im][cur][0].m);
+    m.ax = HM(ax->m);
+    m.wz = PM(S.w[im][cur][1].m);
+    m.az = PM(az->m);
+    m.m1x = PM(S.mu[im][cur][0].m);
+    m.m1z = PM(S.mu[im][cur][1].m);
+    m.mpx = PM(S.mu[im][nx_][0].m);
+    m.mpz = PM(S.mu[im][nx_][1].m);
+    AdjArgs& x = L.a[L.images++];
+    x.c11 = S.c[0].v.origin; x.c13 = S.c[1].v.origin; x.c33 = S.c[2].v.origin;
+    x.d = S.d;
+    x.wz = S.w[im][cur][1].v.origin;
+    x.az = az->v.origin;
+    x.mpx = S.mu[im][nx_][0].v.origin;
+    x.mpz = S.mu[im][nx_][1].v.origin;
+    x.wox = S.w[im][nx_][0].v.origin;
+    x.woz = S.w[im][nx_][1].v.origin;
+    x.g11 = S.img[im][0].v.origin;
+    x.g13 = S.img[im][1].v.origin;
+    x.g33 = S.img[im][2].v.origin;
+    x.dampx = S.damp;
+    x.dampy = S.damp + S.g.nx;
+    x.dampz = S.damp + S.g.nx + S.g.ny;
+    x.sx = dt2 / (S.g.dx * S.g.dx);
+    x.sy = dt2 / (S.g.dy * S.g.dy);
+    x.sz = dt2 / (S.g.dz * S.g.dz);
+    x.status = ctx->d_status;
+  }
+  if (!L.images) return VTI_OK;
+  const Sched sc = make_sched(ctx, S.d, 2, L.images);
+  for (int k = 0; k < L.images; ++k) L.a[k].sc = sc;
   {
     LaunchTimer tm(ctx, kTimedBwd3d);
-    k_adj3d_tma<<<x.sc.grid, NTHREADS, G_SMEM, ctx->stream>>>(m, x);
+    kern<<<sc.grid, NTHREADS, G_SMEM, ctx->stream>>>(L);
   }
   VTI_LAUNCHED(ctx, "k_adj3d_tma");
   return VTI_OK;
@@ -1083,7 +1129,7 @@ int vti3d_gnhv_exact(vti_ctx* ctx, const vti3d_geom* g, const float* c11, const 
   VTI_TRY(store_ck(0, 0));  // a_0 = 0 (buffer 1), a_1 (buffer 0)
   int cur = 0;
   for (int t = 2; t <= M; ++t) {
-    VTI_TRY(launch_born(S, cur, sg, dt2 * wavelet[t - 1]));
+    VTI_TRY(launch_born(S, cur, sg, dt2 * wavelet[t - 1], (t & 1) != 0));
     cur = 1 - cur;  // level t now in `cur`
     if (t < (int)sg.rec_at.size() && sg.rec_at[t] >= 0) {
       VTI_TRY(launch_record(ctx, d_tr, nnt, sg.rec_at[t], S.a[cur][0].v.origin,
@@ -1161,7 +1207,7 @@ int vti3d_gnhv_exact(vti_ctx* ctx, const vti3d_geom* g, const float* c11, const 
       VolM* nx_ = lvl(t);
       VTI_TRY(launch_fwd3d_tma(ctx, S.d, cx[0].m, cx[1].m, px[0].m, px[1].m, S.c[0].m, S.c[1].m,
                                S.c[2].m, cx[1].v.origin, nx_[0].v.origin, nx_[1].v.origin, &dmp,
-                               sxs, sys, szs, ps, Probe(), true));
+                               sxs, sys, szs, ps, Probe(), true, (t & 1) != 0));
       if (b16) {
         const int sl = t - (k0 - 1);
         VTI_TRY(pack(S, nx_[0], S.segb[2 * sl], t, 0));
@@ -1171,9 +1217,10 @@ int vti3d_gnhv_exact(vti_ctx* ctx, const vti3d_geom* g, const float* c11, const 
     for (int tm1 = k1; tm1 >= k0; --tm1) {
       const int t = tm1 + 1;
       const int slot = tm1 - (k0 - 1);
+      if (!b16) VTI_TRY(launch_adj(S, want, mcur, slot, (t & 1) != 0));
       for (int im = 0; im < 2; ++im) {
         if (!want[im]) continue;
-        VTI_TRY(b16 ? launch_adj_b16(S, im, mcur, slot) : launch_adj(S, im, mcur, slot));
+        if (b16) VTI_TRY(launch_adj_b16(S, im, mcur, slot));
         const int nb = 1 - mcur;  // mu_t / w_t were written there
         if (b16 && t < (int)sg.rec_at.size() && sg.rec_at[t] >= 0 && sg.nr > 0) {
           k_inject_exact_b16<<<(sg.nr + 127) / 128, 128, 0, ctx->stream>>>(

@@ -234,7 +234,7 @@ __global__ void k_boundary_merge(Dims3 d, int npad, const float* full, const flo
 // the lags four at a time: sixteen FMAs per level on one new float4 of R (the
 // row is reused from L1) and one float4 of the image per lag.
 // 150x120x80, 32 lags each side: 156 us per level for the one-level kernel,
-// 31 us per level for this one.
+// 28 us per level for this one.
 __device__ __forceinline__ float4 odcig_row4(const float* row, int x, int pitch) {
   return x >= 0 && x < pitch ? __ldg(reinterpret_cast<const float4*>(row + x))
                              : make_float4(0.f, 0.f, 0.f, 0.f);

@@ -103,37 +103,6 @@ __device__ __forceinline__ void model_pair(const float* c11, const float* c13, c
   a33 = any ? __ldg(reinterpret_cast<const float2*>(c33 + i)) : zero;
 }
 
-// March direction. kDir = 1 walks every item down z as numbered; kDir = -1
-// walks the items in reverse order and each item from its last plane to its
-// first. A time loop alternates the two, so a level starts on the planes the
-// level before it touched last, while they are still in L2 (126 MB): a level
-// that always starts at plane 0 finds nothing of a volume set larger than L2
-// there. Every point is computed by the same operations in either direction.
-// Measured, one direction -> alternating (nt 400): gradient 251x203x150 94.6 ->
-// 89.2 ms, 400x400x200 360 -> 350 ms, RTM 256x224x128 61.1 -> 56.5 ms; no
-// change where a level's volumes fit L2 (128^3 modeling 15.5 ms).
-template <int kDir>
-__device__ __forceinline__ int march_item(int i, int items) {
-  return kDir > 0 ? i : items - 1 - i;
-}
-
-// z queue of one x pair: q[j] holds plane z - 4 + j; `in` is plane z + 4
-// (kDir > 0) or z - 4. (Nine unrolled copies of the plane loop with rotating
-// slots save the moves but spill: 482 ms per 400x400x200 gradient of 399
-// levels against 350.)
-template <int kDir>
-__device__ __forceinline__ void queue_shift(float2 (&q)[9], float2 in) {
-  if (kDir > 0) {
-#pragma unroll
-    for (int kk = 0; kk < 8; ++kk) q[kk] = q[kk + 1];
-    q[8] = in;
-  } else {
-#pragma unroll
-    for (int kk = 8; kk > 0; --kk) q[kk] = q[kk - 1];
-    q[0] = in;
-  }
-}
-
 // The sponge's block order (abc3d.cu:82-126): the z stencil reads the planes of
 // the 4-plane blocks above its own already damped. Marching down z, the queue
 // entries of a block are damped once, after its last plane (z; entries 1..4 are
@@ -802,12 +771,12 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 constexpr long long kRestart = 1;
 constexpr int kSegPlanes = 8, kSegPlanesOneWave = 4;
 
-Sched make_sched(vti_ctx* ctx, const Dims3& d, int ctas_per_sm) {
+Sched make_sched(vti_ctx* ctx, const Dims3& d, int ctas_per_sm, int copies) {
   Sched s;
   s.gx = (d.nx - kHalo + TX - 1) / TX;  // x origins 0, 32, ...; updated x < nx-4
   s.gy = (d.ny - 2 * kHalo + TY - 1) / TY;
   s.nz = d.nz;
-  const long long cols = (long long)s.gx * s.gy;
+  const long long cols = (long long)s.gx * s.gy * copies;
   const long long slots = (long long)ctx->sm_count * ctas_per_sm;
   long long best = -1;
   for (int nseg = 1; nseg <= d.nz; ++nseg) {
@@ -822,10 +791,10 @@ Sched make_sched(vti_ctx* ctx, const Dims3& d, int ctas_per_sm) {
     if (best < 0 || cost < best) {
       best = cost;
       s.seg = seg;
-      s.items = (int)items;
+      s.items = (int)(items / copies);
     }
   }
-  s.grid = (int)std::min<long long>(s.items, slots);
+  s.grid = (int)std::min<long long>((long long)s.items * copies, slots);
   return s;
 }
 
