@@ -7,6 +7,10 @@
 // The taper multiplies cur and next after every step (kernels.cu:304-315);
 // stored values here are the once-tapered levels, prev is read as taper*prev.
 //
+// Traces run several levels per launch (vti_tile2d.cu) or, many shots of a small
+// grid at once, resident in one cluster each (below); the per-step path, used for
+// snapshots, the allocation-free form and what those two do not take:
+//
 // One fused kernel per time step: stencil + source + taper; receivers are
 // recorded by a small gather kernel. The source amplitudes of all steps are
 // uploaded once, so every step's launch differs only in its buffer pointers.

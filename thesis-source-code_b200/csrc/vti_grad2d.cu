@@ -2,6 +2,10 @@
 // and Gauss-Newton Hessian-vector product (GNhessian_f, hessian_f.cu:575-1010)
 // for sm_100a.
 //
+// The gradient of receivers and sources in the update region runs several levels
+// per launch (grad2d_tiles, vti_tile2d.cu); what follows is the per-level path of
+// the Gauss-Newton product and of the other gradients.
+//
 // Forward: one fused kernel per level (background; with the Born field and
 // its scattering source for the GN product), checkpoints D(sigma) = (Dxx p,
 // Dzz q) of the levels the backward pass reads, kept on the device.

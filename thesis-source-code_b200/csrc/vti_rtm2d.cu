@@ -1,6 +1,9 @@
 // 2D reverse-time migration (rtm_f, lib/vti-fwi-2d/rtm_f.cu:13-267) for
 // sm_100a.
 //
+// Migrations whose receivers (and the row below them) lie in the update region
+// run several levels per launch (rtm2d_tiles, vti_tile2d.cu); the per-level path:
+//
 // One step kernel serves both wavefields; both are forwardCD levels
 // (kernels.cu:452-498) with the taper of cur and next folded in as in the
 // forward-modeling kernel (stored levels are once-tapered, prev is read as

@@ -8,7 +8,9 @@
 // the owned cells' work, on SMs that would otherwise wait), and writes its own
 // cells of the last two levels into the other of two wavefield sets. Launches
 // follow one another as programmatic dependents; every cell is computed by the
-// operations of the per-level kernels, so results do not depend on the split.
+// operations of the per-level kernels, so results do not depend on the split (the
+// per-level migration injects with global float atomics, which flush subnormal
+// contributions; here they are added).
 //
 // Whole calls, B200, one launch per level -> now: traces 801x401 + 30 cells, 1000
 // levels, three shots 24.0 -> 10.3 ms; traces 201x101 + 30 (one cluster before) 2.30

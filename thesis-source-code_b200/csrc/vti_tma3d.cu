@@ -14,8 +14,8 @@
 // Pipeline. Warp 8 (producer) issues, for every plane of its range, TMA tile
 // loads (cp.async.bulk.tensor.3d, no multicast) of all input planes into a
 // ring of shared-memory stages: the current sigma_x (and lambda_x) plane with
-// a 4-cell halo, the sigma_z (lambda_z) plane 4 below for the register queue,
-// prev, c11/c13/c33 and, in the backward kernel, the gradient tiles. Each
+// a 4-cell halo, the sigma_z (lambda_z) plane 4 ahead for the register queue and
+// prev (the model and the gradients are read by the consumers). Each
 // stage completes on an mbarrier with a transaction count; consumers (warps
 // 0-7, two rows each) release a stage with one arrive per warp. Out-of-range
 // tiles at the far x/y edges are zero-filled by the TMA unit.
