@@ -65,3 +65,42 @@ def test_tiled_gradient_and_migration_match_per_level(ctx, nx, nz, pad, nt, rate
                                      s.taper))
     assert np.abs(a).max() > 0
     assert rel_l2(b, a) < 1e-5
+
+
+@pytest.mark.parametrize("kind,room", [("synthetic", 60), ("gradient", 180), ("migration", 100)])
+def test_calls_run_where_the_tiles_have_no_room(kind, room):
+    """The tiles' padded arrays (131 x 91 cells in 192 x 136) need about twice the
+    memory of the other paths: with `room` MB free the tiles do not fit and the
+    call runs all the same. Levels kept: 250 MB padded, 114 MB not (gradient), 125 and
+    57 MB (migration); 100 shots side by side 94 MB, one after another 2 MB."""
+    import torch
+    synth = kind == "synthetic"
+    s = S.survey2d(nx=111, nz=71, nt=41 if synth else 1201, npad=10, rate=1e-3, ns=100 if synth else 1)
+    a = (s.c11, s.c13, s.c33, s.wavelet, s.sloc, s.rloc, s.taper)
+    small = V.Context(0)
+    try:
+        g = s.geom()
+        data = np.random.default_rng(3).standard_normal(s.nt * (s.rloc.size // 2)).astype(np.float32)
+        call = {"synthetic": lambda c: [V.synthetic_f(c, g, *a)],
+                "gradient": lambda c: V.objFuncGradient_f(c, g, data, *a),
+                "migration": lambda c: [V.rtm_f(c, g, data, *a)]}[kind]
+        warm = V.Context(0)  # loads every kernel while there is room
+        try:
+            tiled = call(warm)
+            warm.set_2d_resident(False)
+            ref = call(warm)
+        finally:
+            warm.close()
+        torch.cuda.empty_cache()
+        torch.cuda.synchronize()
+        hold = torch.empty(torch.cuda.mem_get_info()[0] - (room << 20), dtype=torch.uint8, device="cuda")
+        try:
+            out = call(small)
+        finally:
+            del hold
+            torch.cuda.empty_cache()
+        for x, y, t in zip(out, ref, tiled):
+            assert np.abs(x).max() > 0
+            assert rel_l2(x, y) < 1e-5 and rel_l2(t, y) < 1e-5
+    finally:
+        small.close()

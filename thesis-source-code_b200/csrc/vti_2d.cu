@@ -789,7 +789,7 @@ int synth2d_resident(vti_ctx* ctx, const vti2d_geom* g, const float* c11, const 
 // shots of a chunk (wavefields up to 256 MB) advance together, each into its own
 // traces, which are copied out in shot order (a later shot overwrites the
 // receivers it shares with an earlier one, as in synthetic_f.cu:31-124).
-// VTI_ERR_UNSUPPORTED: not eligible, nothing was computed.
+// VTI_ERR_UNSUPPORTED: not eligible or no room, nothing was computed.
 int synth2d_tiles(vti_ctx* ctx, const vti2d_geom* g, const float* c11, const float* c13,
                   const float* c33, const float* wavelet, const int* sloc, int ns, const int* rloc,
                   int nr_total, const float* taper, float* out) {
@@ -842,6 +842,7 @@ int synth2d_tiles(vti_ctx* ctx, const vti2d_geom* g, const float* c11, const flo
   float *flat, *model, *waves, *d_amp, *d_data;
   int *d_map, *d_row, *d_src, *d_nri, *d_cells;
   long long* d_off;
+  CallBlock mem;
   float* buf = nullptr;
   for (int pass = 0; pass < 2; ++pass) {
     tile2d::Carve c{reinterpret_cast<char*>(buf)};
@@ -856,7 +857,7 @@ int synth2d_tiles(vti_ctx* ctx, const vti2d_geom* g, const float* c11, const flo
     d_off = c.take<long long>(ns);
     d_cells = c.take<int>(std::max<size_t>(cells.size(), 1));
     d_data = c.take<float>(std::max<long long>(n_data, 1));
-    if (pass == 0) VTI_TRY_RES(scratch2d(ctx, c.used, &buf));
+    if (pass == 0 && !(buf = mem.get(ctx, c.used))) return VTI_ERR_UNSUPPORTED;
   }
   cudaStream_t s = ctx->stream;
   // margins and frame of the model stay zero

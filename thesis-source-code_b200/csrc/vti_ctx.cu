@@ -185,21 +185,49 @@ int vol_download(vti_ctx* ctx, const Dims3& d, const Vol* v, float* dst, int mem
   return rows_download(ctx, d, v->origin, dst, mem);
 }
 
+namespace {
+void drop_scratch2d(vti_ctx* ctx) {
+  if (ctx->scratch2d) {
+    cudaStreamSynchronize(ctx->stream);
+    cudaFree(ctx->scratch2d);
+  }
+  ctx->scratch2d = nullptr;
+  ctx->scratch2d_bytes = 0;
+}
+}  // namespace
+
 // The context's 2D scratch, grown (never shrunk) to `bytes`; freed with the
 // context.
 int scratch2d(vti_ctx* ctx, size_t bytes, float** out) {
   if (ctx->scratch2d_bytes < bytes) {
-    if (ctx->scratch2d) {
-      VTI_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-      cudaFree(ctx->scratch2d);
-      ctx->scratch2d = nullptr;
-      ctx->scratch2d_bytes = 0;
-    }
+    drop_scratch2d(ctx);
     VTI_CUDA(ctx, cudaMalloc((void**)&ctx->scratch2d, bytes));
     ctx->scratch2d_bytes = bytes;
   }
   *out = ctx->scratch2d;
   return VTI_OK;
+}
+
+float* CallBlock::get(vti_ctx* ctx, size_t bytes) {
+  if (ctx->scratch2d_bytes >= bytes) return ctx->scratch2d;
+  const bool keep = bytes <= kScratch2dKeep;
+  if (keep) drop_scratch2d(ctx);
+  float* p = nullptr;
+  if (cudaMalloc((void**)&p, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    drop_scratch2d(ctx);
+    if (keep || cudaMalloc((void**)&p, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+  }
+  if (keep) {
+    ctx->scratch2d = p;
+    ctx->scratch2d_bytes = bytes;
+  } else {
+    own = p;
+  }
+  return p;
 }
 
 int check_device_status(vti_ctx* ctx) {

@@ -370,7 +370,7 @@ struct Buf {
 // The gradient through the tiled kernels (vti_tile2d.cu): receivers of a shot in
 // the update region and on different cells, sources in it as well. The same
 // levels, checkpoints and injections as run_grad2d. VTI_ERR_UNSUPPORTED: not
-// eligible, nothing was computed.
+// eligible or no room, nothing was computed.
 int grad2d_tiles(vti_ctx* ctx, const vti2d_geom* g, float* gc11, float* gc13, float* gc33,
                  const float* data, const float* c11, const float* c13, const float* c33,
                  const float* wavelet, const int* sloc, int ns, const int* rloc, int nr,
@@ -398,7 +398,7 @@ int grad2d_tiles(vti_ctx* ctx, const vti2d_geom* g, float* gc11, float* gc13, fl
   double* d_acc;
   unsigned char* live;
   tile2d::BackLevel* d_lv;
-  Buf own;  // a block larger than the context keeps
+  CallBlock mem;
   float* block = nullptr;
   for (int pass = 0; pass < 2; ++pass) {
     tile2d::Carve c{reinterpret_cast<char*>(block)};
@@ -421,13 +421,8 @@ int grad2d_tiles(vti_ctx* ctx, const vti2d_geom* g, float* gc11, float* gc13, fl
     live = c.take<unsigned char>(nnt_data);
     d_lv = c.take<tile2d::BackLevel>(nt);
     if (pass) break;
-    if (c.used <= kScratch2dKeep) {
-      const int st = scratch2d(ctx, c.used, &block);
-      if (st != VTI_OK) return st;
-    } else {
-      VTI_CUDA(ctx, cudaMalloc((void**)&own.p, c.used));
-      block = own.p;
-    }
+    block = mem.get(ctx, c.used);
+    if (!block) return VTI_ERR_UNSUPPORTED;
   }
   cudaStream_t s = ctx->stream;
   VTI_CUDA(ctx, cudaMemsetAsync(model, 0, 4 * L.n * sizeof(float), s));

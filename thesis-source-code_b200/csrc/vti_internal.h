@@ -161,11 +161,25 @@ int cuda_check(vti_ctx* ctx, cudaError_t e, const char* what);
   } while (0)
 
 // The context's 2D scratch of at least `bytes` bytes (kept between calls, freed
-// with the context). Gradients and migrations use it up to kScratch2dKeep, which a
-// 461 x 261 gradient of 1800 levels reaches, and allocate per call beyond: one of
-// 590 MB costs 1 to 4 ms of a 6 ms call in cudaMalloc and cudaFree.
-constexpr size_t kScratch2dKeep = (size_t)1 << 30;
+// with the context).
 int scratch2d(vti_ctx* ctx, size_t bytes, float** out);
+// Device memory of one call of the tiled 2D forms: the context's scratch up to
+// kScratch2dKeep, which a 461 x 261 gradient of 1800 levels reaches (allocating and
+// freeing 590 MB costs 1 to 4 ms of a 6 ms call), beyond that a block of its own,
+// freed with this. get returns null, and leaves no error behind, when the device
+// has no room even without the scratch: the caller then takes the per-level path,
+// which needs less.
+constexpr size_t kScratch2dKeep = (size_t)1 << 30;
+struct CallBlock {
+  float* own = nullptr;
+  float* get(vti_ctx* ctx, size_t bytes);
+  CallBlock() = default;
+  CallBlock(const CallBlock&) = delete;
+  CallBlock& operator=(const CallBlock&) = delete;
+  ~CallBlock() {
+    if (own) cudaFree(own);
+  }
+};
 
 int vol_alloc(vti_ctx* ctx, const Dims3& d, Vol* v);
 void vol_free(Vol* v);

@@ -153,7 +153,7 @@ namespace {
 // rtm_f through the tiled kernels (vti_tile2d.cu): receivers of a shot, with the
 // row below them, in the update region and on different cells. The same levels,
 // slices and injections as rtm2d_impl, which has checked the arguments.
-// VTI_ERR_UNSUPPORTED: not eligible, nothing was computed.
+// VTI_ERR_UNSUPPORTED: not eligible or no room, nothing was computed.
 int rtm2d_tiles(vti_ctx* ctx, const vti2d_geom* g, float* image, const float* data,
                 const float* c11, const float* c13, const float* c33, const float* wavelet,
                 const int* sloc, int ns, const int* rloc, int nr, const float* taper) {
@@ -172,12 +172,7 @@ int rtm2d_tiles(vti_ctx* ctx, const vti2d_geom* g, float* image, const float* da
   float *flat, *model, *waves, *img, *slices, *ddata, *d_amp;
   int *d_map, *d_keep, *d_src, *d_cells;
   tile2d::BackLevel* d_lv;
-  struct Block {  // larger than the context keeps
-    float* p = nullptr;
-    ~Block() {
-      if (p) cudaFree(p);
-    }
-  } own;
+  CallBlock mem;
   float* block = nullptr;
   const size_t n_data = (size_t)std::max(nnt_data, 0) * nr;
   for (int pass = 0; pass < 2; ++pass) {
@@ -195,13 +190,8 @@ int rtm2d_tiles(vti_ctx* ctx, const vti2d_geom* g, float* image, const float* da
     d_cells = c.take<int>(std::max(nr, 1));
     d_lv = c.take<tile2d::BackLevel>(nt);
     if (pass) break;
-    if (c.used <= kScratch2dKeep) {
-      const int st = scratch2d(ctx, c.used, &block);
-      if (st != VTI_OK) return st;
-    } else {
-      VTI_CUDA(ctx, cudaMalloc((void**)&own.p, c.used));
-      block = own.p;
-    }
+    block = mem.get(ctx, c.used);
+    if (!block) return VTI_ERR_UNSUPPORTED;
   }
   cudaStream_t s = ctx->stream;
   VTI_CUDA(ctx, cudaMemsetAsync(model, 0, 4 * L.n * sizeof(float), s));
