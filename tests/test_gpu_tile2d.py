@@ -104,3 +104,32 @@ def test_calls_run_where_the_tiles_have_no_room(kind, room):
             assert rel_l2(x, y) < 1e-5 and rel_l2(t, y) < 1e-5
     finally:
         small.close()
+
+
+def test_many_shots_on_shared_receivers(ctx):
+    """1000 shots, each on 200 receivers of which the next shots record most again
+    (the last one to record a receiver stands): several chunks of shots, traces equal
+    to one shot after another, and device memory of a chunk, not of the 320 MB of all
+    shots' traces beside it."""
+    import torch
+    s = S.survey2d(nx=220, nz=60, nt=400, npad=10, rate=1e-3)
+    ns, nri = 1000, 200
+    s.rloc = np.array([[10 + (7 * k) % 220, 11 + k // 220] for k in range(1100)], np.int32).reshape(-1)
+    s.sloc = np.array([[14 + (5 * k) % 210, 12, nri, (37 * k) % 900] for k in range(ns)],
+                      np.int32).reshape(-1)
+    a = (s.geom(), s.c11, s.c13, s.c33, s.wavelet, s.sloc, s.rloc, s.taper)
+    own = V.Context(0)
+    try:
+        V.synthetic_f(own, a[0], *a[1:5], s.sloc[:4], s.rloc, s.taper)  # loads the kernels
+        before = torch.cuda.mem_get_info()[0]
+        out = V.synthetic_f(own, *a)
+        assert before - torch.cuda.mem_get_info()[0] < 300 << 20
+    finally:
+        own.close()
+    ctx.set_2d_resident(False)
+    try:
+        ref = V.synthetic_f(ctx, *a)
+    finally:
+        ctx.set_2d_resident(True)
+    assert np.abs(ref).max() > 0
+    assert np.array_equal(out, ref)

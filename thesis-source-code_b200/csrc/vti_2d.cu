@@ -786,9 +786,10 @@ int synth2d_resident(vti_ctx* ctx, const vti2d_geom* g, const float* c11, const 
 
 // Traces of all shots through the tiled kernel (vti_tile2d.cu): every source in
 // the update region, the receivers of a shot in it and on different cells. The
-// shots of a chunk (wavefields up to 256 MB) advance together, each into its own
-// traces, which are copied out in shot order (a later shot overwrites the
-// receivers it shares with an earlier one, as in synthetic_f.cu:31-124).
+// shots of a chunk (256 MB of wavefields and traces) advance together, each into
+// its own traces, which are copied out in shot order (a later shot overwrites the
+// receivers it shares with an earlier one, as in synthetic_f.cu:31-124). Shots whose
+// receivers are the whole list in order write the caller's array as it is.
 // VTI_ERR_UNSUPPORTED: not eligible or no room, nothing was computed.
 int synth2d_tiles(vti_ctx* ctx, const vti2d_geom* g, const float* c11, const float* c13,
                   const float* c33, const float* wavelet, const int* sloc, int ns, const int* rloc,
@@ -816,8 +817,6 @@ int synth2d_tiles(vti_ctx* ctx, const vti2d_geom* g, const float* c11, const flo
   cover = cover && next == nr_total;
   VTI_CUDA(ctx, cudaSetDevice(ctx->device));
   const tile2d::Layout L = tile2d::make_layout(ctx, nnx, nnz, ns, false);
-  const size_t per_shot = (tile2d::kWaveArrays + 1) * L.n * sizeof(float);
-  const int chunk = (int)std::max<size_t>(1, std::min<size_t>(ns, ((size_t)256 << 20) / per_shot));
   // trace row taken at each level, -1 none, and the source term of each level
   std::vector<int> row(g->nt, -1);
   if (ratio == 1 && g->ot == 0.f) row[1] = 1;
@@ -827,18 +826,30 @@ int synth2d_tiles(vti_ctx* ctx, const vti2d_geom* g, const float* c11, const flo
     if (t >= 0.f && (it - ntNeg) % ratio == 0) row[it] = (it - ntNeg) / ratio;
     amp[it] = dt2 * wavelet[it - 1];
   }
-  std::vector<int> src(ns), nri(ns), cells;
-  std::vector<long long> off(ns);
-  long long n_data = 0;
+  std::vector<int> src(ns), nri(ns), cells, first;  // first: of each chunk, and ns
+  std::vector<long long> off(ns);  // of a shot's traces in the block of its chunk
+  constexpr size_t kChunkBytes = (size_t)256 << 20;
+  long long n_data = cover ? nrows * nr_total : 0, in_chunk = 0;
+  int chunk = 0;  // shots of the largest chunk
   for (int is = 0; is < ns; ++is) {
     const int* sh = sloc + 4 * is;
+    const size_t waves_bytes = (tile2d::kWaveArrays + 1) * L.n * sizeof(float);
+    const long long recs = cover ? 0 : nrows * sh[2];
+    if (first.empty() || (is + 1 - first.back()) * waves_bytes +
+                                 (size_t)(in_chunk + recs) * sizeof(float) > kChunkBytes) {
+      first.push_back(is);
+      in_chunk = 0;
+    }
     src[is] = L.at(sh[0], sh[1]);
     nri[is] = cover ? nr_total : sh[2];
-    off[is] = cover ? sh[3] : n_data;
-    n_data += nrows * sh[2];
+    off[is] = cover ? sh[3] : in_chunk;
+    in_chunk += recs;
+    n_data = std::max(n_data, in_chunk);
+    chunk = std::max(chunk, is + 1 - first.back());
     for (int ir = 0; ir < sh[2]; ++ir)
       cells.push_back(L.at(rloc[2 * (sh[3] + ir)], rloc[2 * (sh[3] + ir) + 1]));
   }
+  first.push_back(ns);
   float *flat, *model, *waves, *d_amp, *d_data;
   int *d_map, *d_row, *d_src, *d_nri, *d_cells;
   long long* d_off;
@@ -876,7 +887,6 @@ int synth2d_tiles(vti_ctx* ctx, const vti2d_geom* g, const float* c11, const flo
   VTI_CUDA(ctx, up(d_nri, nri.data(), ns * sizeof(int)));
   VTI_CUDA(ctx, up(d_off, off.data(), ns * sizeof(long long)));
   VTI_CUDA(ctx, up(d_cells, cells.data(), cells.size() * sizeof(int)));
-  VTI_CUDA(ctx, cudaMemsetAsync(d_data, 0, std::max<long long>(n_data, 1) * sizeof(float), s));
   tile2d::Forward f{};
   f.L = L;
   f.m = {model, model + L.n, model + 2 * L.n, model + 3 * L.n, 1.f / (g->dx * g->dx),
@@ -886,8 +896,11 @@ int synth2d_tiles(vti_ctx* ctx, const vti2d_geom* g, const float* c11, const flo
   f.rec_row = d_row;
   f.rec = d_data;
   size_t cell0 = 0;
-  for (int is0 = 0; is0 < ns; is0 += chunk) {
-    f.shots = std::min(chunk, ns - is0);
+  for (size_t c = 0; c + 1 < first.size(); ++c) {
+    const int is0 = first[c];
+    f.shots = first[c + 1] - is0;
+    if (c == 0 || !cover)
+      VTI_CUDA(ctx, cudaMemsetAsync(d_data, 0, std::max<long long>(n_data, 1) * sizeof(float), s));
     VTI_CUDA(ctx, cudaMemsetAsync(waves, 0, f.shots * f.wave_stride * sizeof(float), s));
     for (int k = 0; k < f.shots; ++k) {
       const int* sh = sloc + 4 * (is0 + k);
@@ -918,17 +931,15 @@ int synth2d_tiles(vti_ctx* ctx, const vti2d_geom* g, const float* c11, const flo
       VTI_TRY_RES(tile2d::launch_forward(ctx, f));
       std::swap(in, other);
     }
+    if (!cover)
+      for (int is = is0; is < first[c + 1]; ++is)
+        if (nri[is] > 0)
+          VTI_CUDA(ctx, cudaMemcpy2DAsync(out + sloc[4 * is + 3], (size_t)nr_total * 4,
+                                          d_data + off[is], (size_t)nri[is] * 4,
+                                          (size_t)nri[is] * 4, nrows, cudaMemcpyDeviceToHost, s));
   }
-  if (cover) {
-    if (n_data)
-      VTI_CUDA(ctx, cudaMemcpyAsync(out, d_data, n_data * sizeof(float), cudaMemcpyDeviceToHost, s));
-  } else {
-    for (int is = 0; is < ns; ++is)
-      if (nri[is] > 0)
-        VTI_CUDA(ctx, cudaMemcpy2DAsync(out + sloc[4 * is + 3], (size_t)nr_total * 4,
-                                        d_data + off[is], (size_t)nri[is] * 4, (size_t)nri[is] * 4,
-                                        nrows, cudaMemcpyDeviceToHost, s));
-  }
+  if (cover && n_data)
+    VTI_CUDA(ctx, cudaMemcpyAsync(out, d_data, n_data * sizeof(float), cudaMemcpyDeviceToHost, s));
   VTI_CUDA(ctx, cudaStreamSynchronize(s));
   return VTI_OK;
 }
