@@ -129,3 +129,19 @@ def test_resident_traces_equal_per_step_traces(ctx, kw):
         ctx.set_2d_resident(True)
     assert np.abs(step).max() > 0
     np.testing.assert_array_equal(res, step)
+
+
+@pytest.mark.parametrize("nx,nz,ns", [(97, 37, 1), (97, 37, 3), (401, 201, 1)])
+def test_receivers_outside_the_grid_are_refused_whatever_the_path(ctx, nx, nz, ns):
+    """Grids that fit one cluster: a receiver outside the grid is refused even if no
+    shot records it, whether the cluster or the tiles would run the call."""
+    s = S.survey2d(nx=nx, nz=nz, nt=60, npad=10, ns=ns)
+    rloc = np.concatenate([s.rloc, np.array([nx + 20, 5], np.int32)])  # first column outside
+    args = (ctx, s.geom(), s.c11, s.c13, s.c33, s.wavelet, s.sloc)
+    with pytest.raises(V.VtiError, match="outside the grid"):
+        V.synthetic_f(*args, rloc, s.taper)
+    ctx.set_2d_resident(False)
+    try:  # the per-level path reads only the receivers of the shots
+        V.synthetic_f(*args, rloc, s.taper)
+    finally:
+        ctx.set_2d_resident(True)

@@ -673,6 +673,21 @@ int run2d(vti_ctx* ctx, const vti2d_geom* g, const float* c11, const float* c13,
   return VTI_OK;
 }
 
+// Whether one cluster per shot can run this call: a grid that fits one, sources
+// in the update region, a valid record.
+bool resident_takes(vti_ctx* ctx, const vti2d_geom* g, const int* sloc, int ns, ResShape* shape) {
+  const int nnx = g->nx + 2 * g->npad, nnz = g->nz + 2 * g->npad;
+  if (!ctx->resident2d || ns < 1 || nnx < 9 || nnz < 9 || g->nt < 2 || !(g->dt > 0) ||
+      !(g->rate > 0) || (int)(g->rate / g->dt + 0.5f) < 1)
+    return false;
+  for (int is = 0; is < ns; ++is) {
+    const int* sh = sloc + 4 * is;
+    if (sh[0] < kHalo || sh[0] >= nnx - kHalo || sh[1] < kHalo || sh[1] >= nnz - kHalo)
+      return false;
+  }
+  return cudaSetDevice(ctx->device) == cudaSuccess && resident_shape(ctx, nnx, nnz, shape);
+}
+
 // Traces of all shots of a grid that fits one thread-block cluster
 // (resident_shape) with every source in the update region: the model is
 // uploaded once and each shot runs in its own cluster of k_synth2d_resident
@@ -684,27 +699,12 @@ int run2d(vti_ctx* ctx, const vti2d_geom* g, const float* c11, const float* c13,
 int synth2d_resident(vti_ctx* ctx, const vti2d_geom* g, const float* c11, const float* c13,
                      const float* c33, const float* wavelet, const int* sloc, int ns,
                      const int* rloc, int nr_total, const float* taper, float* out) {
-  if (!ctx->resident2d || ns < 1) return VTI_ERR_UNSUPPORTED;
   const int nnx = g->nx + 2 * g->npad, nnz = g->nz + 2 * g->npad;
   const long long nnxz = (long long)nnx * nnz;
-  if (nnx < 9 || nnz < 9 || g->nt < 2 || !(g->dt > 0) || !(g->rate > 0))
-    return VTI_ERR_UNSUPPORTED;
-  for (int is = 0; is < ns; ++is) {
-    const int* sh = sloc + 4 * is;
-    if (sh[0] < kHalo || sh[0] >= nnx - kHalo || sh[1] < kHalo || sh[1] >= nnz - kHalo)
-      return VTI_ERR_UNSUPPORTED;
-  }
+  ResShape shape;
+  if (!resident_takes(ctx, g, sloc, ns, &shape)) return VTI_ERR_UNSUPPORTED;
   const float dt = g->dt, dt2 = dt * dt;
   const int ratio = (int)(g->rate / dt + 0.5f);
-  if (ratio < 1) return VTI_ERR_UNSUPPORTED;
-  VTI_CUDA(ctx, cudaSetDevice(ctx->device));
-  ResShape shape;
-  if (!resident_shape(ctx, nnx, nnz, &shape)) return VTI_ERR_UNSUPPORTED;
-  for (int ir = 0; ir < nr_total; ++ir) {
-    const int x = rloc[2 * ir], z = rloc[2 * ir + 1];
-    if (x < 0 || x >= nnx || z < 0 || z >= nnz)
-      return fail(ctx, VTI_ERR_ARG, "2D receiver outside the grid");
-  }
   const int ntNeg = (int)std::round(std::fabs(g->ot) / dt);
   // trace row taken at each level, -1 none (the arithmetic of run2d)
   std::vector<int> hi(g->nt, -1);
@@ -984,6 +984,16 @@ int vti2d_synthetic(vti_ctx* ctx, const vti2d_geom* g, const float* c11, const f
   }
   if (!c11 || !c13 || !c33 || !wavelet || !taper || !data) return VTI_ERR_ARG;
   VTI_TRY_RES(check_cfl2d(ctx, g, c11, c13, c33));
+  // A call that a cluster can run is refused for any receiver of the list outside
+  // the grid, whichever way it goes then; the per-level path looks at the receivers
+  // that a shot records.
+  ResShape shape;
+  if (resident_takes(ctx, g, sloc, ns, &shape)) {
+    const int nnz = g->nz + 2 * g->npad;
+    for (int ir = 0; ir < nr; ++ir)
+      if (rloc[2 * ir] < 0 || rloc[2 * ir] >= nnx || rloc[2 * ir + 1] < 0 || rloc[2 * ir + 1] >= nnz)
+        return fail(ctx, VTI_ERR_ARG, "2D receiver outside the grid");
+  }
   const bool tiles = tiles_faster(ctx, g, sloc, ns);
   for (int k = 0; k < 2; ++k) {  // the faster way first, the other if it cannot take the call
     const int st = (k == 0) == tiles
