@@ -145,3 +145,30 @@ def test_receivers_outside_the_grid_are_refused_whatever_the_path(ctx, nx, nz, n
         V.synthetic_f(*args, rloc, s.taper)
     finally:
         ctx.set_2d_resident(True)
+
+
+@pytest.mark.parametrize("nx,nz,nt,ns,cluster", [
+    (41, 31, 200, 1, True),     # 101 x 91: a cluster's level is shorter
+    (201, 101, 10, 1, True),    # 261 x 161, a short record: the tiles' preparation costs more
+    (201, 101, 1000, 1, False),
+    (201, 101, 500, 4, True),   # four shots fill the GPU either way
+    (401, 201, 500, 14, True),  # 461 x 261, 16 CTAs of 16 rows, more shots than clusters
+    (401, 201, 500, 2, False)])
+def test_cluster_or_tiles_by_cost(ctx, nx, nz, nt, ns, cluster):
+    """Shots on receivers of their own run where they take less time: one launch with
+    a cluster per shot, or tiles; the traces are those of the per-step path."""
+    s = S.survey2d(nx=nx, nz=nz, nt=nt, ns=ns)
+    sl = s.sloc.reshape(-1, 4)
+    sl[:, 2] = nx // ns
+    sl[:, 3] = np.arange(ns) * (nx // ns)
+    args = (ctx, s.geom(), s.c11, s.c13, s.c33, s.wavelet, s.sloc, s.rloc, s.taper)
+    before = ctx.launches
+    res = V.synthetic_f(*args)
+    assert (ctx.launches - before == 1) == cluster
+    ctx.set_2d_resident(False)
+    try:
+        step = V.synthetic_f(*args)
+    finally:
+        ctx.set_2d_resident(True)
+    assert nt < 100 or np.abs(step).max() > 0
+    np.testing.assert_array_equal(res, step)

@@ -694,15 +694,12 @@ bool resident_takes(vti_ctx* ctx, const vti2d_geom* g, const int* sloc, int ns, 
 // (all levels in shared memory). Shots whose receiver ranges are disjoint
 // share one launch; otherwise one launch per shot, in shot order, so a later
 // shot overwrites the receivers it shares with an earlier one (the per-shot
-// order of synthetic_f.cu:31-124). VTI_ERR_UNSUPPORTED: not eligible, the
-// caller runs the per-level path (nothing was computed).
-int synth2d_resident(vti_ctx* ctx, const vti2d_geom* g, const float* c11, const float* c13,
-                     const float* c33, const float* wavelet, const int* sloc, int ns,
-                     const int* rloc, int nr_total, const float* taper, float* out) {
+// order of synthetic_f.cu:31-124). shape: resident_takes's, the receivers checked.
+int synth2d_resident(vti_ctx* ctx, const ResShape& shape, const vti2d_geom* g, const float* c11,
+                     const float* c13, const float* c33, const float* wavelet, const int* sloc,
+                     int ns, const int* rloc, int nr_total, const float* taper, float* out) {
   const int nnx = g->nx + 2 * g->npad, nnz = g->nz + 2 * g->npad;
   const long long nnxz = (long long)nnx * nnz;
-  ResShape shape;
-  if (!resident_takes(ctx, g, sloc, ns, &shape)) return VTI_ERR_UNSUPPORTED;
   const float dt = g->dt, dt2 = dt * dt;
   const int ratio = (int)(g->rate / dt + 0.5f);
   const int ntNeg = (int)std::round(std::fabs(g->ot) / dt);
@@ -945,17 +942,17 @@ int synth2d_tiles(vti_ctx* ctx, const vti2d_geom* g, const float* c11, const flo
 }
 
 // Whether the tiled kernel is the faster way for these shots. It spreads a shot
-// over all SMs; a cluster keeps one on up to 16 SMs without launches, at about
-// 1.4 us per level plus 0.25 us per 1000 cells of an SM (measured 2.0 us at 261 x
-// 161, 3.2 us at 461 x 261; the tiles take 1.6 and 1.75), and runs as many shots at
-// once as there are clusters, if their receivers are disjoint: 14 shots of 461 x
-// 261 take 8.4 us per level there and 15 us in tiles.
-bool tiles_faster(vti_ctx* ctx, const vti2d_geom* g, const int* sloc, int ns) {
+// over all SMs, a launch of several levels at a time (make_layout has its cost); a
+// cluster keeps one on up to 16 SMs without launches, at about 1.35 us per level plus
+// 0.29 us per 1000 cells of an SM (measured 1.31 us at 101 x 91, 1.67 at 181 x 121, 2.12
+// at 261 x 161, 3.3 at 461 x 261; the tiles take 1.61, 1.58, 1.65 and 1.85), and runs as
+// many shots at once as there are clusters, if their receivers are disjoint: 261 x
+// 161, four shots 2.25 us per level there and 2.38 in tiles; 461 x 261, 14 shots 7.1 and
+// 15.4. Before the first level the tiles lay out the padded arrays and, per shot, the
+// receiver map: 35 us and 7 us per shot more (five levels of 101 x 91 107 against 80
+// us, of 16 shots of 261 x 161 435 against 295), which short records do not earn back.
+bool tiles_faster(vti_ctx* ctx, const ResShape& shape, const vti2d_geom* g, const int* sloc, int ns) {
   const int nnx = g->nx + 2 * g->npad, nnz = g->nz + 2 * g->npad;
-  ResShape shape;
-  if (nnx < 9 || nnz < 9 || ns < 1 || cudaSetDevice(ctx->device) != cudaSuccess ||
-      !resident_shape(ctx, nnx, nnz, &shape))
-    return true;
   std::vector<std::pair<int, int>> rng;
   for (int is = 0; is < ns; ++is) rng.push_back({sloc[4 * is + 3], sloc[4 * is + 3] + sloc[4 * is + 2]});
   std::sort(rng.begin(), rng.end());
@@ -965,7 +962,7 @@ bool tiles_faster(vti_ctx* ctx, const vti2d_geom* g, const int* sloc, int ns) {
   const double cells = (double)(nnx - 2 * kHalo) * shape.rows;
   double tiles = 0;
   tile2d::make_layout(ctx, nnx, nnz, ns, false, &tiles);
-  return tiles < rounds * (1.4 + 0.25e-3 * cells);
+  return 35 + 7.0 * ns + g->nt * tiles < g->nt * rounds * (1.35 + 0.29e-3 * cells);
 }
 
 }  // namespace
@@ -988,20 +985,19 @@ int vti2d_synthetic(vti_ctx* ctx, const vti2d_geom* g, const float* c11, const f
   // the grid, whichever way it goes then; the per-level path looks at the receivers
   // that a shot records.
   ResShape shape;
-  if (resident_takes(ctx, g, sloc, ns, &shape)) {
+  const bool cluster = resident_takes(ctx, g, sloc, ns, &shape);
+  if (cluster) {
     const int nnz = g->nz + 2 * g->npad;
     for (int ir = 0; ir < nr; ++ir)
       if (rloc[2 * ir] < 0 || rloc[2 * ir] >= nnx || rloc[2 * ir + 1] < 0 || rloc[2 * ir + 1] >= nnz)
         return fail(ctx, VTI_ERR_ARG, "2D receiver outside the grid");
   }
-  const bool tiles = tiles_faster(ctx, g, sloc, ns);
-  for (int k = 0; k < 2; ++k) {  // the faster way first, the other if it cannot take the call
-    const int st = (k == 0) == tiles
-                       ? synth2d_tiles(ctx, g, c11, c13, c33, wavelet, sloc, ns, rloc, nr, taper, data)
-                       : synth2d_resident(ctx, g, c11, c13, c33, wavelet, sloc, ns, rloc, nr, taper,
-                                          data);
+  if (!cluster || tiles_faster(ctx, shape, g, sloc, ns)) {
+    const int st = synth2d_tiles(ctx, g, c11, c13, c33, wavelet, sloc, ns, rloc, nr, taper, data);
     if (st != VTI_ERR_UNSUPPORTED) return st;
   }
+  if (cluster)
+    return synth2d_resident(ctx, shape, g, c11, c13, c33, wavelet, sloc, ns, rloc, nr, taper, data);
   for (int is = 0; is < ns; ++is) {
     const int* s = sloc + 4 * is;
     int st = run2d(ctx, g, c11, c13, c33, wavelet, taper, s[0] + s[1] * nnx, rloc, s[2], nr, s[3],

@@ -495,13 +495,11 @@ std::atomic<bool> attr_fwd[2][kMaxT + 1][64], attr_bwd[2][kMaxT + 1][64];
 
 }  // namespace
 
-// A launch takes about 3.4 + 0.85 T us per wave of one CTA per SM (forward;
-// measured T = 2..5: 4.9, 5.9, 6.3, 7.4 us over 4 to 14 waves of three 861 x 461
-// grids, 6.5, 7.1, 8.0 us for T = 3..5 on the 261 x 161 grid that fits one wave): the
-// first part is loading the square, so more levels per launch pay while the
-// smaller tiles still fit the waves. 1000 levels, T = 2 / 3 / 4 / 5: 261 x 161 one
-// shot - / 2.37 / 1.96 / 1.83 ms, 861 x 461 three shots 10.7 / 12.4 / 14.4 / 21.0 ms,
-// gradient 461 x 261 - / 7.4 / 6.2 / 8.8 ms.
+// A launch takes about 0.5 us and 3.4 + 0.85 T us per wave of one CTA per SM: the
+// first part of a wave is loading the square, so more levels per launch pay while
+// the smaller tiles still fit the waves. Forward, us per launch for T = 2 / 3 / 4 / 5:
+// one wave (28 to 77 CTAs, 261 x 161) 5.3 / 6.5 / 7.1 / 8.2, two waves (112 to 209 CTAs, 461 x
+// 261) 5.5 / 6.8 / 7.4 / 15.4, 4 to 14 waves (three shots of 861 x 461) 19.4 / 34.9 / 55 / 101.
 Layout make_layout(vti_ctx* ctx, int nnx, int nnz, int shots, bool backward, double* us_per_level) {
   Layout best;
   double cost = 0;
@@ -518,7 +516,8 @@ Layout make_layout(vti_ctx* ctx, int nnx, int nnz, int shots, bool backward, dou
     L.W = ((L.ntx - 1) * L.tile + kExt + 31) & ~31;
     L.n = (size_t)L.W * ((L.ntz - 1) * L.tile + kExt);
     const long long ctas = (long long)L.ntx * L.ntz * shots;
-    const double c = (double)((ctas + ctx->sm_count - 1) / ctx->sm_count) * (3.4 + 0.85 * T) / T;
+    const double c =
+        (0.5 + (double)((ctas + ctx->sm_count - 1) / ctx->sm_count) * (3.4 + 0.85 * T)) / T;
     if (!best.T || c < cost) {
       best = L;
       cost = c;
