@@ -133,3 +133,26 @@ def test_many_shots_on_shared_receivers(ctx):
         ctx.set_2d_resident(True)
     assert np.abs(ref).max() > 0
     assert np.array_equal(out, ref)
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+@pytest.mark.parametrize("nx,nz", [(57, 30), (60, 60)])
+def test_nonfinite_samples_spread_as_per_level(ctx, value, nx, nz):
+    """A NaN or infinite observed sample makes the same cells of gradient and image
+    NaN as one launch per level does; the frame that no step updates stays zero."""
+    s = S.survey2d(nx=nx, nz=nz, nt=62, npad=12, rate=2e-3)
+    s = shots(s, [12 + nx // 2], nx // 3, nz + 14)  # receivers near the far side
+    data = np.random.default_rng(2).standard_normal((31, nx // 3)).astype(np.float32)
+    data[20, 5] = value
+    nnx, nnz = nx + 24, nz + 24
+    for call in (lambda: V.objFuncGradient_f(ctx, s.geom(), data, s.c11, s.c13, s.c33, s.wavelet,
+                                             s.sloc, s.rloc, s.taper)[:3],
+                 lambda: [V.rtm_f(ctx, s.geom(), data, s.c11, s.c13, s.c33, s.wavelet, s.sloc,
+                                  s.rloc, s.taper)]):
+        for x, y in zip(*both(ctx, call)):
+            x, y = x.reshape(nnz, nnx), y.reshape(nnz, nnx)
+            assert np.isnan(x).any() and np.isfinite(x).any()
+            assert np.array_equal(np.isnan(x), np.isnan(y)) and np.array_equal(np.isinf(x), np.isinf(y))
+            frame = np.ones((nnz, nnx), bool)
+            frame[4:-4, 4:-4] = False
+            assert not y[frame].any()

@@ -873,7 +873,7 @@ int synth2d_tiles(vti_ctx* ctx, const vti2d_geom* g, const float* c11, const flo
   const float* host[4] = {c11, c13, c33, taper};
   for (int k = 0; k < 4; ++k) {
     VTI_CUDA(ctx, cudaMemcpyAsync(flat, host[k], nnxz * sizeof(float), cudaMemcpyHostToDevice, s));
-    VTI_TRY_RES(tile2d::launch_pad(ctx, L, flat, model + k * L.n, true));
+    VTI_TRY_RES(tile2d::launch_pad(ctx, L, flat, model + k * L.n));
   }
   auto up = [&](void* d, const void* h, size_t bytes) {
     return bytes ? cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s) : cudaSuccess;

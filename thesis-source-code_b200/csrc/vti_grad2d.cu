@@ -429,7 +429,7 @@ int grad2d_tiles(vti_ctx* ctx, const vti2d_geom* g, float* gc11, float* gc13, fl
   const float* host[4] = {c11, c13, c33, taper};
   for (int k = 0; k < 4; ++k) {
     VTI_CUDA(ctx, cudaMemcpyAsync(flat, host[k], nnxz * sizeof(float), cudaMemcpyHostToDevice, s));
-    const int st = tile2d::launch_pad(ctx, L, flat, model + k * L.n, true);
+    const int st = tile2d::launch_pad(ctx, L, flat, model + k * L.n);
     if (st != VTI_OK) return st;
   }
   VTI_CUDA(ctx, cudaMemsetAsync(grad, 0, 3 * L.n * sizeof(float), s));

@@ -199,7 +199,7 @@ int rtm2d_tiles(vti_ctx* ctx, const vti2d_geom* g, float* image, const float* da
   int st = VTI_OK;
   for (int k = 0; k < 4 && st == VTI_OK; ++k) {
     VTI_CUDA(ctx, cudaMemcpyAsync(flat, host[k], nnxz * sizeof(float), cudaMemcpyHostToDevice, s));
-    st = tile2d::launch_pad(ctx, L, flat, model + k * L.n, true);
+    st = tile2d::launch_pad(ctx, L, flat, model + k * L.n);
   }
   if (st != VTI_OK) return st;
   if (n_data)

@@ -437,17 +437,17 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 // ------------------------------------------------------------ small kernels
+// kPad: into the padded layout, otherwise out of it; zero in the outer lo cells of
+// the grid (the padded frame at the far sides is owned by tiles and, though its
+// fields are zero times whatever its neighbours hold, NaN beside a NaN).
 template <bool kPad>
 __global__ void k_pad(Layout L, const float* src, float* dst, int lo) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= L.nnx * L.nnz) return;
-  const int x = i % L.nnx, z = i / L.nnx;
-  if (!kPad) {
-    dst[i] = src[L.at(x, z)];
-    return;
-  }
+  const int x = i % L.nnx, z = i / L.nnx, j = L.at(x, z);
   const bool in = x >= lo && x < L.nnx - lo && z >= lo && z < L.nnz - lo;
-  dst[L.at(x, z)] = in ? src[i] : 0.f;
+  const float v = in ? src[kPad ? i : j] : 0.f;
+  dst[kPad ? j : i] = v;
 }
 
 __global__ void k_map(const int* cells, int n, int* map) {
@@ -567,15 +567,15 @@ int launch_backward(vti_ctx* ctx, const Backward& a) {
   return VTI_OK;
 }
 
-int launch_pad(vti_ctx* ctx, const Layout& L, const float* src, float* dst, bool core) {
+int launch_pad(vti_ctx* ctx, const Layout& L, const float* src, float* dst) {
   const int n = L.nnx * L.nnz;
-  k_pad<true><<<(n + 255) / 256, 256, 0, ctx->stream>>>(L, src, dst, core ? kHalo : 0);
+  k_pad<true><<<(n + 255) / 256, 256, 0, ctx->stream>>>(L, src, dst, kHalo);
   VTI_LAUNCHED(ctx, "k_pad");
   return VTI_OK;
 }
 int launch_unpad(vti_ctx* ctx, const Layout& L, const float* src, float* dst) {
   const int n = L.nnx * L.nnz;
-  k_pad<false><<<(n + 255) / 256, 256, 0, ctx->stream>>>(L, src, dst, 0);
+  k_pad<false><<<(n + 255) / 256, 256, 0, ctx->stream>>>(L, src, dst, kHalo);
   VTI_LAUNCHED(ctx, "k_unpad");
   return VTI_OK;
 }

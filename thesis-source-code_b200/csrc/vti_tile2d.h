@@ -93,8 +93,9 @@ struct Backward {
 };
 int launch_backward(vti_ctx* ctx, const Backward& a);
 
-// Contiguous nnx x nnz array into the padded layout; core: only the update region.
-int launch_pad(vti_ctx* ctx, const Layout& L, const float* src, float* dst, bool core);
+// Contiguous nnx x nnz array into the padded layout and back: the update region,
+// zeros in the frame around it.
+int launch_pad(vti_ctx* ctx, const Layout& L, const float* src, float* dst);
 int launch_unpad(vti_ctx* ctx, const Layout& L, const float* src, float* dst);
 // map[cell] = receiver for the given padded cells, -1 elsewhere.
 int launch_map(vti_ctx* ctx, const Layout& L, const int* cells, int n, int* map);
