@@ -813,7 +813,8 @@ int synth2d_tiles(vti_ctx* ctx, const vti2d_geom* g, const float* c11, const flo
   }
   cover = cover && next == nr_total;
   VTI_CUDA(ctx, cudaSetDevice(ctx->device));
-  const tile2d::Layout L = tile2d::make_layout(ctx, nnx, nnz, ns, false);
+  const tile2d::Layout L = tile2d::make_layout(ctx->sm_count, nnx, nnz, ns, false);
+  if (!L.T) return VTI_ERR_UNSUPPORTED;
   // trace row taken at each level, -1 none, and the source term of each level
   std::vector<int> row(g->nt, -1);
   if (ratio == 1 && g->ot == 0.f) row[1] = 1;
@@ -961,7 +962,7 @@ bool tiles_faster(vti_ctx* ctx, const ResShape& shape, const vti2d_geom* g, cons
   const int rounds = disjoint ? (ns + shape.clusters - 1) / shape.clusters : ns;
   const double cells = (double)(nnx - 2 * kHalo) * shape.rows;
   double tiles = 0;
-  tile2d::make_layout(ctx, nnx, nnz, ns, false, &tiles);
+  tile2d::make_layout(ctx->sm_count, nnx, nnz, ns, false, &tiles);
   return 35 + 7.0 * ns + g->nt * tiles < g->nt * rounds * (1.35 + 0.29e-3 * cells);
 }
 

@@ -389,7 +389,8 @@ int grad2d_tiles(vti_ctx* ctx, const vti2d_geom* g, float* gc11, float* gc13, fl
     max_nri = std::max(max_nri, sl[2]);
   }
   const float dt = g->dt, dt2 = dt * dt;
-  const tile2d::Layout L = tile2d::make_layout(ctx, nnx, nnz, 1, true);
+  const tile2d::Layout L = tile2d::make_layout(ctx->sm_count, nnx, nnz, 1, true);
+  if (!L.T) return VTI_ERR_UNSUPPORTED;
   const int zero = (int)slot.size();  // one more checkpoint, of zeros
   const size_t nrec = (size_t)nnt_data * max_nri;
   float *flat, *model, *waves, *grad, *kept, *rec, *obs, *d_amp;

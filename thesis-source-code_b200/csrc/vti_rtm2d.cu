@@ -167,7 +167,8 @@ int rtm2d_tiles(vti_ctx* ctx, const vti2d_geom* g, float* image, const float* da
   const int ratio = (int)(g->rate / dt + 0.5f);
   const int ntNeg = (int)std::round(std::fabs(g->ot) / dt);
   const int nnt = (nt - 1) / ratio + 1, nnt_data = (nt - ntNeg - 1) / ratio + 1;
-  const tile2d::Layout L = tile2d::make_layout(ctx, nnx, nnz, 1, true);
+  const tile2d::Layout L = tile2d::make_layout(ctx->sm_count, nnx, nnz, 1, true);
+  if (!L.T) return VTI_ERR_UNSUPPORTED;
   VTI_CUDA(ctx, cudaSetDevice(ctx->device));
   float *flat, *model, *waves, *img, *slices, *ddata, *d_amp;
   int *d_map, *d_keep, *d_src, *d_cells;

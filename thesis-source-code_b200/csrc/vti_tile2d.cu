@@ -35,7 +35,6 @@ constexpr int kThreads = 512, kRows = 4, kWarps = kThreads / 32;
 static_assert(kWarps * kRows == kExt && kExt == 64, "one warp per four rows");
 static_assert(kHalo == kRows, "a level drops one warp (and two lanes) at each end");
 
-constexpr int kMinT = 2, kMaxT = 5;  // levels per launch
 constexpr int kField = kExt * kExt;             // floats
 constexpr int kGuard = 8;                       // reads of x - 4 in row 0, x + 5 in the last
 constexpr int kFieldsSmem = 4 * kField + 2 * kGuard;
@@ -494,38 +493,6 @@ std::atomic<bool> attr_fwd[2][kMaxT + 1][64], attr_bwd[2][kMaxT + 1][64];
   } while (0)
 
 }  // namespace
-
-// A launch takes about 0.5 us and 3.4 + 0.85 T us per wave of one CTA per SM: the
-// first part of a wave is loading the square, so more levels per launch pay while
-// the smaller tiles still fit the waves. Forward, us per launch for T = 2 / 3 / 4 / 5:
-// one wave (28 to 77 CTAs, 261 x 161) 5.3 / 6.5 / 7.1 / 8.2, two waves (112 to 209 CTAs, 461 x
-// 261) 5.5 / 6.8 / 7.4 / 15.4, 4 to 14 waves (three shots of 861 x 461) 19.4 / 34.9 / 55 / 101.
-Layout make_layout(vti_ctx* ctx, int nnx, int nnz, int shots, bool backward, double* us_per_level) {
-  Layout best;
-  double cost = 0;
-  // two levels' D pairs and images of 48 x 48 cells do not fit shared memory
-  for (int T = backward ? 3 : kMinT; T <= kMaxT; ++T) {
-    Layout L;
-    L.nnx = nnx;
-    L.nnz = nnz;
-    L.T = T;
-    L.tile = kExt - 2 * kHalo * T;
-    L.off = kHalo * T - kHalo;
-    L.ntx = (nnx - 2 * kHalo + L.tile - 1) / L.tile;
-    L.ntz = (nnz - 2 * kHalo + L.tile - 1) / L.tile;
-    L.W = ((L.ntx - 1) * L.tile + kExt + 31) & ~31;
-    L.n = (size_t)L.W * ((L.ntz - 1) * L.tile + kExt);
-    const long long ctas = (long long)L.ntx * L.ntz * shots;
-    const double c =
-        (0.5 + (double)((ctas + ctx->sm_count - 1) / ctx->sm_count) * (3.4 + 0.85 * T)) / T;
-    if (!best.T || c < cost) {
-      best = L;
-      cost = c;
-    }
-  }
-  if (us_per_level) *us_per_level = cost;
-  return best;
-}
 
 int launch_forward(vti_ctx* ctx, const Forward& a) {
   using Kernel = void (*)(Forward);

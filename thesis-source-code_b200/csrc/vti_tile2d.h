@@ -9,7 +9,8 @@
 namespace vti {
 namespace tile2d {
 
-constexpr int kExt = 64;  // cells per side that a CTA holds
+constexpr int kExt = 64;           // cells per side that a CTA holds
+constexpr int kMinT = 2, kMaxT = 5;  // levels per launch
 
 // How a grid is cut: T levels per launch, so a CTA owns the inner tile = 64 - 8 T
 // cells per side of the 64 it holds. Every array is padded: grid cell (x, z) at
@@ -21,9 +22,42 @@ struct Layout {
   __host__ __device__ int at(int x, int z) const { return x + off + (z + off) * W; }
 };
 // The layout for `shots` grids advanced side by side (backward: by the backward
-// kernel too); *us_per_level: what a forward level of all of them takes.
-Layout make_layout(vti_ctx* ctx, int nnx, int nnz, int shots, bool backward,
-                   double* us_per_level = nullptr);
+// kernel too) on sm_count SMs; *us_per_level: what a forward level of all of them
+// takes. T = 0: a grid so thin and long that its padded arrays pass the 2^31 cells
+// that an index counts, or that a launch's second dimension passes 65535 tiles.
+//
+// A launch takes about 0.5 us and 3.4 + 0.85 T us per wave of one CTA per SM: the
+// first part of a wave is loading the square, so more levels per launch pay while
+// the smaller tiles still fit the waves. Forward, us per launch for T = 2 / 3 / 4 / 5:
+// one wave (28 to 77 CTAs, 261 x 161) 5.3 / 6.5 / 7.1 / 8.2, two waves (112 to 209 CTAs, 461 x
+// 261) 5.5 / 6.8 / 7.4 / 15.4, 4 to 14 waves (three shots of 861 x 461) 19.4 / 34.9 / 55 / 101.
+inline Layout make_layout(int sm_count, int nnx, int nnz, int shots, bool backward,
+                          double* us_per_level = nullptr) {
+  Layout best;
+  double cost = 0;
+  // two levels' D pairs and images of 48 x 48 cells do not fit shared memory
+  for (int T = backward ? 3 : kMinT; T <= kMaxT; ++T) {
+    Layout L;
+    L.nnx = nnx;
+    L.nnz = nnz;
+    L.T = T;
+    L.tile = kExt - 2 * kHalo * T;
+    L.off = kHalo * T - kHalo;
+    L.ntx = (nnx - 2 * kHalo + L.tile - 1) / L.tile;
+    L.ntz = (nnz - 2 * kHalo + L.tile - 1) / L.tile;
+    L.W = ((L.ntx - 1) * L.tile + kExt + 31) & ~31;
+    L.n = (size_t)L.W * ((L.ntz - 1) * L.tile + kExt);
+    if (L.n > 0x7fffffff || L.ntz > 65535) continue;
+    const long long ctas = (long long)L.ntx * L.ntz * shots;
+    const double c = (0.5 + (double)((ctas + sm_count - 1) / sm_count) * (3.4 + 0.85 * T)) / T;
+    if (!best.T || c < cost) {
+      best = L;
+      cost = c;
+    }
+  }
+  if (us_per_level) *us_per_level = cost;
+  return best;
+}
 
 // Model arrays in the padded layout, zero outside the update region (so a level
 // needs no bounds tests: next = taper * (...) is 0 there, as in the frame).
