@@ -499,7 +499,7 @@ int launch_forward(vti_ctx* ctx, const Forward& a) {
   static const Kernel kerns[2][kMaxT + 1] = {
       {nullptr, nullptr, k_tile_forward<false, 2>, k_tile_forward<false, 3>,
        k_tile_forward<false, 4>, k_tile_forward<false, 5>},
-      {nullptr, nullptr, k_tile_forward<true, 2>, k_tile_forward<true, 3>, k_tile_forward<true, 4>,
+      {nullptr, nullptr, nullptr, k_tile_forward<true, 3>, k_tile_forward<true, 4>,
        k_tile_forward<true, 5>}};
   const int fused = a.keep_mode != kKeepNone;  // the gradient's and migration's arithmetic
   constexpr int bytes = kFieldsSmem * sizeof(float);
@@ -517,10 +517,10 @@ int launch_forward(vti_ctx* ctx, const Forward& a) {
 int launch_backward(vti_ctx* ctx, const Backward& a) {
   using Kernel = void (*)(Backward);
   static const Kernel kerns[2][kMaxT + 1] = {
-      {nullptr, nullptr, k_tile_backward<false, 2>, k_tile_backward<false, 3>,
-       k_tile_backward<false, 4>, k_tile_backward<false, 5>},
-      {nullptr, nullptr, nullptr, k_tile_backward<true, 3>,
-       k_tile_backward<true, 4>, k_tile_backward<true, 5>}};
+      {nullptr, nullptr, nullptr, k_tile_backward<false, 3>, k_tile_backward<false, 4>,
+       k_tile_backward<false, 5>},
+      {nullptr, nullptr, nullptr, k_tile_backward<true, 3>, k_tile_backward<true, 4>,
+       k_tile_backward<true, 5>}};
   const int bytes =
       (a.exact ? BackSmem<true>::floats(a.L.T) : BackSmem<false>::floats(a.L.T)) * sizeof(float);
   const Kernel kern = kerns[a.exact ? 1 : 0][a.L.T];

@@ -10,7 +10,7 @@ namespace vti {
 namespace tile2d {
 
 constexpr int kExt = 64;           // cells per side that a CTA holds
-constexpr int kMinT = 2, kMaxT = 5;  // levels per launch
+constexpr int kMinT = 2, kMinBackT = 3, kMaxT = 5;  // levels per launch
 
 // How a grid is cut: T levels per launch, so a CTA owns the inner tile = 64 - 8 T
 // cells per side of the 64 it holds. Every array is padded: grid cell (x, z) at
@@ -31,12 +31,19 @@ struct Layout {
 // the smaller tiles still fit the waves. Forward, us per launch for T = 2 / 3 / 4 / 5:
 // one wave (28 to 77 CTAs, 261 x 161) 5.3 / 6.5 / 7.1 / 8.2, two waves (112 to 209 CTAs, 461 x
 // 261) 5.5 / 6.8 / 7.4 / 15.4, 4 to 14 waves (three shots of 861 x 461) 19.4 / 34.9 / 55 / 101.
+// A gradient's two launches together take about 1 us and 12.6 + 0.85 T us per wave
+// (T = 3 / 4 / 5: 461 x 261 16.3 / 17.2 / 34.7 us, 1061 x 561 46 / 71 / 133), a migration's 1.5
+// us and 8.6 + 1.45 T (15.1 / 16.1 / 31.9, 39.5 / 68 / 125). Choosing their depth by those
+// gives the same one as the forward cost for every grid of 190..861 x 130..461, so one
+// rule serves all.
 inline Layout make_layout(int sm_count, int nnx, int nnz, int shots, bool backward,
                           double* us_per_level = nullptr) {
   Layout best;
   double cost = 0;
-  // two levels' D pairs and images of 48 x 48 cells do not fit shared memory
-  for (int T = backward ? 3 : kMinT; T <= kMaxT; ++T) {
+  // backward from 3: the D pairs of two levels and their images and the gradient's
+  // images of 48 x 48 cells do not fit shared memory (a migration's one image and two
+  // slices would; its kernels are built for the same depths)
+  for (int T = backward ? kMinBackT : kMinT; T <= kMaxT; ++T) {
     Layout L;
     L.nnx = nnx;
     L.nnz = nnz;
