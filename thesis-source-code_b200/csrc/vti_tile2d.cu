@@ -83,7 +83,7 @@ __device__ __forceinline__ float2 carry(float2 cur, float2 t, float2 prev) {
 template <bool kFused, int T>
 __global__ void __launch_bounds__(kThreads, 1) k_tile_forward(const __grid_constant__ Forward a) {
   pdl_launch_next();
-  extern __shared__ float sm_raw[];
+  extern __shared__ __align__(16) float sm_raw[];
   float* sm = sm_raw + kGuard;  // [x field 0][z field 0][x field 1][z field 1]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int W = a.L.W, r0 = warp * kRows, c0 = 2 * lane;
@@ -231,6 +231,11 @@ struct BackSmem {
   __host__ __device__ static constexpr int floats(int T) {
     return kImage + (kImages + (T + 1) * kKept) * (kExt - 2 * kHalo * T) * (kExt - 2 * kHalo * T);
   }
+  // 16-byte copies into the kept arrays: every piece before them and every row of a
+  // tile (8 (8 - T) floats) is a multiple of four floats
+  static_assert(kTaper % 4 == 0 && kC13 % 4 == 0 && kImage % 4 == 0 && (2 * kHalo) % 4 == 0 &&
+                    kExt % 4 == 0,
+                "16-byte pieces");
 };
 
 // The kept arrays of level `lv` over the owned cells into buf: [a][b] (exact:
@@ -258,7 +263,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     k_tile_backward(const __grid_constant__ Backward a) {
   using S = BackSmem<kExact>;
   pdl_launch_next();
-  extern __shared__ float sm_raw[];
+  extern __shared__ __align__(16) float sm_raw[];
   float* sm = sm_raw + kGuard;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int W = a.L.W, r0 = warp * kRows, c0 = 2 * lane;
