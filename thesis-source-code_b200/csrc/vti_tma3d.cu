@@ -895,8 +895,10 @@ std::atomic<bool> attr_fwd[8][64], attr_bwd[4][64], attr_fwd_batch[2][64], attr_
 // to another SM, and half of the time to the other die's L2, from one level to
 // the next: 2 % on 400x400x200 and 251x203x150 gradients, whose launches last
 // 50 us and more. Hence only launches that move at most 250 MB (about 40 us).
-// With few CTAs (80x80x64: 120) early CTAs share SMs that others leave empty
-// (model 2.84 -> 3.24 ms over 299 levels): at least 1.5 per SM.
+// With few CTAs early ones share SMs that others leave empty, and nothing is gained
+// (64^3, 128 CTAs, 299 levels: model 2.05 against 2.11 ms early, gradient 7.02 against 6.97);
+// from 1.5 per SM on it pays (80x80x64, 240 CTAs: model 2.34 -> 2.17 ms, gradient 7.93 ->
+// 7.14; 110x97x83 3.27 -> 2.49 and 10.7 -> 9.1).
 static bool early_launch(vti_ctx* ctx, const Dims3& d, int bytes_per_point, int grid) {
   return d.npoints() * bytes_per_point <= 250000000LL && 2 * grid >= 3 * ctx->sm_count;
 }
