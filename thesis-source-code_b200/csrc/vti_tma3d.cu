@@ -758,44 +758,8 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   return fn;
 }
 
-// Segment length: the smallest modelled time, counted in plane-steps of one
-// CTA, waves * (seg + restart), where a wave is one item per resident slot
-// and a restart (8 queue planes read with plain loads, pipeline refill) costs
-// about kRestart plane-steps. Segments of fewer than 8 planes (down to 4) only
-// while all items are resident at once: there they fill slots that would idle,
-// with more waves they only add restarts.
-// Measured with the alternating march (nt 300..514), restart 4 -> 1: gradient
-// 300x200x90 50.3 -> 46.8 ms, 251x203x150 89.4 -> 87.9, 400x400x200 and
-// 128^3..208x192x128 unchanged; short segments: 110x97x83 one-call 22.7 -> 20.4 ms,
-// 112x112x96 12.2 -> 11.7 ms, allowed everywhere 160x160x112 25.0 -> 25.5 ms.
-constexpr long long kRestart = 1;
-constexpr int kSegPlanes = 8, kSegPlanesOneWave = 4;
-
-Sched make_sched(vti_ctx* ctx, const Dims3& d, int ctas_per_sm, int copies) {
-  Sched s;
-  s.gx = (d.nx - kHalo + TX - 1) / TX;  // x origins 0, 32, ...; updated x < nx-4
-  s.gy = (d.ny - 2 * kHalo + TY - 1) / TY;
-  s.nz = d.nz;
-  const long long cols = (long long)s.gx * s.gy * copies;
-  const long long slots = (long long)ctx->sm_count * ctas_per_sm;
-  long long best = -1;
-  for (int nseg = 1; nseg <= d.nz; ++nseg) {
-    const int seg = (d.nz + nseg - 1) / nseg;
-    if (nseg > 1 && seg < kSegPlanesOneWave) break;
-    if (nseg > 1 && seg == (d.nz + nseg - 2) / (nseg - 1)) continue;  // same seg
-    const long long items = cols * ((d.nz + seg - 1) / seg);
-    if (items > (1LL << 30)) break;
-    const long long waves = (items + slots - 1) / slots;
-    if (nseg > 1 && seg < kSegPlanes && waves > 1) continue;
-    const long long cost = waves * (seg + kRestart);
-    if (best < 0 || cost < best) {
-      best = cost;
-      s.seg = seg;
-      s.items = (int)(items / copies);
-    }
-  }
-  s.grid = (int)std::min<long long>((long long)s.items * copies, slots);
-  return s;
+Sched make_sched(vti_ctx* ctx, const Dims3& d, int ctas_per_sm, int copies, long long launch_planes) {
+  return plan_sched(ctx->sm_count, d, ctas_per_sm, copies, launch_planes);
 }
 
 long long step_sched_cost(vti_ctx* ctx, const Dims3& d, int ctas_per_sm, long long* work) {
@@ -1014,10 +978,13 @@ int fwd_batch_build(vti_ctx* ctx, const FwdJobSpec* spec, int njobs, StepBatch**
     FwdBatch& B = b->fb.back();
     std::memset(&B, 0, sizeof(B));
     std::vector<FwdMaps> maps(2 * nj);
+    long long planes = 0;
+    for (int j = 0; j < nj; ++j) planes += sched_columns(spec[j0 + j].d) * spec[j0 + j].d.nz;
     int items = 0;
     for (int j = 0; j < nj; ++j) {
       const FwdJobSpec& sp = spec[j0 + j];
-      const Sched sc = sp.seg > 0 ? sched_with_seg(sp.d, sp.seg) : make_sched(ctx, sp.d, 3);
+      const Sched sc = sp.seg > 0 ? sched_with_seg(sp.d, sp.seg)
+                                  : make_sched(ctx, sp.d, 3, 1, planes);
       PointSource src;
       src.x = sp.src_x; src.y = sp.src_y; src.z = sp.src_z;
       B.c[j] = fwd_common(sp.d, sc, sp.damp, sp.sx, sp.sy, sp.sz, src, *sp.c[0], *sp.c[1],
@@ -1064,10 +1031,13 @@ int bwd_batch_build(vti_ctx* ctx, const BwdJobSpec* spec, int njobs, StepBatch**
     BwdBatch& B = b->bb.back();
     std::memset(&B, 0, sizeof(B));
     std::vector<BwdMaps> maps(2 * nj);
+    long long planes = 0;
+    for (int j = 0; j < nj; ++j) planes += sched_columns(spec[j0 + j].d) * spec[j0 + j].d.nz;
     int items = 0;
     for (int j = 0; j < nj; ++j) {
       const BwdJobSpec& sp = spec[j0 + j];
-      const Sched sc = sp.seg > 0 ? sched_with_seg(sp.d, sp.seg) : make_sched(ctx, sp.d, 2);
+      const Sched sc = sp.seg > 0 ? sched_with_seg(sp.d, sp.seg)
+                                  : make_sched(ctx, sp.d, 2, 1, planes);
       BwdCommon& c = B.c[j];
       c.d = sp.d;
       c.sc = sc;

@@ -11,23 +11,16 @@
 
 #include "vti_internal.h"
 #include "vti_pair.cuh"
+#include "vti_sched.h"
 
 namespace vti {
-
-struct Sched {
-  int gx, gy;  // columns in x, y
-  int nz;
-  int seg;     // planes per segment
-  int items;   // gx * gy * ceil(nz / seg)
-  int grid;    // persistent CTAs, min(items, resident slots)
-};
 
 namespace {
 
 constexpr float kC0 = -2.84722222222f, kC1 = 1.6f, kC2 = -0.2f, kC3 = 0.02539682539f,
                 kC4 = -0.00178571428f;
 
-constexpr int TX = 32, TY = 16, RY = 2, NCW = TY / RY;  // consumer warps
+constexpr int RY = 2, NCW = TY / RY;  // consumer warps
 constexpr int NTHREADS = (NCW + 1) * 32;
 constexpr int HX = TX + 2 * kHalo, HY = TY + 2 * kHalo;
 // BF16 halo tiles: x from x0-8 so the TMA x coordinate is 16-byte aligned
@@ -201,9 +194,9 @@ __device__ __forceinline__ unsigned char* ring_init(unsigned char* smem_raw, uin
 
 }  // namespace
 
-// Segment schedule of one launch over d with `ctas_per_sm` resident CTAs per SM;
-// copies: the launch works on that many volume sets at once (items per copy).
-Sched make_sched(vti_ctx* ctx, const Dims3& d, int ctas_per_sm, int copies = 1);
+// plan_sched on the context's device.
+Sched make_sched(vti_ctx* ctx, const Dims3& d, int ctas_per_sm, int copies = 1,
+                 long long launch_planes = 0);
 // cuTensorMapEncodeTiled from the driver (null if unavailable).
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn();
 
