@@ -473,12 +473,12 @@ int backward_loop(vti3d_batch* b) {
 }
 
 // Speed of the side-by-side step kernels relative to the single-grid kernels
-// on windows that fill the GPU (whole gradients with the alternating march, six
-// and 16 windows of 160..400 x 160..400 x 200 cells: 0.90 to 0.94; it was 0.79 when
-// both marched one way), and the gap between two single-grid launches in CTA-slot
-// plane-steps (about 3 us; one plane-step of a 32 x 16 column is about 2 us).
-// Windows whose schedule keeps the SMs less busy lose side by side nothing or
-// gain up to 4 % (160x160x150, 224x224x100).
+// on windows that fill the GPU (whole gradients: 16 windows of 160..400 x 160..400 x 200
+// cells 234 against 210 ms, six of them 162 against 160.5), and the gap between two
+// single-grid launches in CTA-slot plane-steps (about 3 us; one plane-step of a
+// 32 x 16 column is about 2 us). Windows whose schedule keeps the SMs less busy gain
+// side by side: six of 224 x 224 x 100 104.6 against 109.1 ms, four of 64..96 x 64..96 x 64
+// 8.9 against 12.8.
 constexpr double kSideBySideRel = 0.9;
 constexpr long long kLaunchGap = 2;
 
@@ -879,29 +879,34 @@ int vti3d_batch_autotune(vti3d_batch* b, int* seg_fwd, int* seg_bwd) {
   }
   VTI_TRY(build_tables(b));
   if (b->schedule == VTI_BATCH_AUTO) {
-    // one level of each schedule (both forward passes, the backward pass and
-    // the receiver work of every shot), timed over `reps` levels after one
-    // untimed level
-    auto side = [&](int t) -> int {
-      VTI_TRY(fwd_tick(b, t));
-      return bwd_tick(b, t);
+    // a few consecutive levels of each pass under each schedule, with the
+    // receiver work, as the gradient runs them: side by side every shot's forward
+    // levels, then the backward ones; per shot one pass after another, on
+    // alternating buffers, so that either finds what its last level left in L2
+    const int lev = std::min(8, M - 1);
+    auto side = [&]() -> int {
+      for (int t = 0; t < lev; ++t) VTI_TRY(fwd_tick(b, t));
+      for (int t = 0; t < lev; ++t) VTI_TRY(bwd_tick(b, t));
+      return VTI_OK;
     };
-    auto per_shot = [&](int) -> int {
+    auto per_shot = [&]() -> int {
       for (size_t k = 0; k < b->plans.size(); ++k) {
         vti3d_plan* p = b->plans[k];
         const ShotGeom& sg = b->geo[k];
-        VTI_TRY(fwd_level(p, sg, true, 0, 1, 2));
-        VTI_TRY(fwd_level(p, sg, false, 0, 1, 2));
-        VTI_TRY(bwd_level(p, sg, false, 0, 1, 0, 1, 0));
+        for (int pass = 0; pass < 2; ++pass)
+          for (int t = 0; t < lev; ++t)
+            VTI_TRY(fwd_level(p, sg, pass == 0, t & 1, 1 - (t & 1), 2 + t));
+        for (int t = 0; t < lev; ++t)
+          VTI_TRY(bwd_level(p, sg, false, t & 1, 1 - (t & 1), t & 1, 1 - (t & 1), t));
       }
       return VTI_OK;
     };
     float t[2] = {0.f, 0.f};
     for (int which = 0; which < 2; ++which) {
-      auto one = [&](int tick) { return which == 0 ? side(tick) : per_shot(tick); };
-      VTI_TRY(one(0));
+      auto run = [&]() { return which == 0 ? side() : per_shot(); };
+      VTI_TRY(run());
       VTI_CUDA(ctx, cudaEventRecord(e0, ctx->stream));
-      for (int r = 0; r < reps; ++r) VTI_TRY(one(r));
+      VTI_TRY(run());
       VTI_CUDA(ctx, cudaEventRecord(e1, ctx->stream));
       VTI_CUDA(ctx, cudaEventSynchronize(e1));
       VTI_CUDA(ctx, cudaEventElapsedTime(&t[which], e0, e1));
