@@ -14,7 +14,7 @@
 
 #include <algorithm>
 #include <cstdint>
-#include <system_error>
+#include <exception>
 #include <thread>
 #include <vector>
 
@@ -59,8 +59,8 @@ class Populate {
               return;
         });
       }
-    } catch (const std::system_error&) {
-      // fewer threads, or none: the copy faults the pages in itself
+    } catch (const std::exception&) {
+      // no thread or no memory for one: the copy faults the other pages in itself
     }
   }
 
