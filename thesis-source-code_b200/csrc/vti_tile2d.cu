@@ -345,9 +345,10 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
       for (int j = 0; j < kRows; ++j) {
         const int o = j * tile;
-        if (kExact) {  // gradientCrossCor (kernels.cu:438-450)
+        if (kExact) {  // gradientCrossCor (kernels.cu:438-450), rounded as in the per-level kernel:
+          // the product that is rounded by itself is f D_b of Dp and (1 - f) D_a of Dq
           const float2 Dp = fma2(g, ld2(d + o), mul2(f2, ld2(d + 2 * kOwned + o)));
-          const float2 Dq = fma2(g, ld2(d + kOwned + o), mul2(f2, ld2(d + 3 * kOwned + o)));
+          const float2 Dq = fma2(f2, ld2(d + 3 * kOwned + o), mul2(g, ld2(d + kOwned + o)));
           st2(img + o, fma2(pc[j], Dp, ld2(img + o)));
           st2(img + kOwned + o, add2(ld2(img + kOwned + o), fma2(qc[j], Dp, mul2(pc[j], Dq))));
           st2(img + 2 * kOwned + o, fma2(qc[j], Dq, ld2(img + 2 * kOwned + o)));
