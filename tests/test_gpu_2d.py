@@ -91,29 +91,32 @@ def test_synthetic_config_size(ctx):
 
 
 @pytest.mark.parametrize("kw", [
-    dict(),  # the benchmark grid: 461 x 261, 16 CTAs of 16 rows, source in exchanged rows
+    dict(),  # the benchmark grid, 461 x 261: one shot runs in tiles
     dict(nx=97, nz=37, nt=240, npad=9, d=10.0, dt=1e-3, rate=1e-3, freq=20.0, src_x=480.0,
-         src_z=120.0, rec_z=0.0, ns=3),  # ragged rows, every step sampled, source in exchanged rows
+         src_z=120.0, rec_z=0.0, ns=3),  # shots on receivers of their own in a cluster each
+    # (ragged rows, every step sampled, source in exchanged rows), on shared ones in tiles
     dict(nx=1100, nz=24, nt=120, npad=8, d=10.0, dt=1e-3, rate=2e-3, freq=15.0, src_x=5000.0,
-         src_z=100.0, rec_z=20.0),  # wider than one cluster: per-step path either way
+         src_z=100.0, rec_z=20.0),  # wider than one cluster: tiles
 ])
 def test_resident_traces_equal_per_step_traces(ctx, kw):
-    """The shared-memory resident launch (one cluster per shot) and the
-    per-step launches compute every point with the same operations: the
+    """The shared-memory resident launch (one cluster per shot), the tiles and
+    the per-step launches compute every point with the same operations: the
     traces are bitwise equal."""
     s = S.survey2d(**kw)
     g = s.geom()
     args = (ctx, g, s.c11, s.c13, s.c33, s.wavelet, s.sloc, s.rloc, s.taper)
     if kw.get("ns", 1) > 1:
         # the survey's shots all record every receiver (a later shot
-        # overwrites: one launch per shot); also run disjoint receiver blocks
-        # (all shots in one launch, one cluster each)
+        # overwrites); also run disjoint receiver blocks (all shots in one
+        # launch, one cluster each)
         sl = s.sloc.reshape(-1, 4).copy()
         nrb = (s.rloc.size // 2) // len(sl)
         sl[:, 2] = nrb
         sl[:, 3] = np.arange(len(sl)) * nrb
         args2 = (ctx, g, s.c11, s.c13, s.c33, s.wavelet, sl.reshape(-1), s.rloc, s.taper)
+        before = ctx.launches
         res2 = V.synthetic_f(*args2)
+        assert ctx.launches - before == 1
         ctx.set_2d_resident(False)
         try:
             step2 = V.synthetic_f(*args2)
@@ -171,4 +174,26 @@ def test_cluster_or_tiles_by_cost(ctx, nx, nz, nt, ns, cluster):
     finally:
         ctx.set_2d_resident(True)
     assert nt < 100 or np.abs(step).max() > 0
+    np.testing.assert_array_equal(res, step)
+
+
+@pytest.mark.parametrize("shared", [False, True])
+def test_cluster_takes_what_the_tiles_refuse(ctx, shared):
+    """Two receivers of a shot on one cell: every shot runs in a cluster, all of them
+    in one launch or, where they share receivers, one launch after another."""
+    s = S.survey2d(nx=97, nz=37, nt=240, npad=9, rate=1e-3, ns=3)
+    sl, rl = s.sloc.reshape(-1, 4), s.rloc.reshape(-1, 2)
+    if not shared:
+        sl[:, 2], sl[:, 3] = 32, np.arange(3) * 32
+    rl[1::32] = rl[0::32][: len(rl[1::32])]
+    args = (ctx, s.geom(), s.c11, s.c13, s.c33, s.wavelet, s.sloc, s.rloc, s.taper)
+    before = ctx.launches
+    res = V.synthetic_f(*args)
+    assert ctx.launches - before == (3 if shared else 1)
+    ctx.set_2d_resident(False)
+    try:
+        step = V.synthetic_f(*args)
+    finally:
+        ctx.set_2d_resident(True)
+    assert np.abs(step).max() > 0
     np.testing.assert_array_equal(res, step)

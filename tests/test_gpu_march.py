@@ -14,8 +14,13 @@ import vtib200.synth as S
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nx,ny,nz,npad", [(40, 36, 24, 6), (41, 25, 21, 5), (33, 37, 26, 7),
-                                           (70, 26, 35, 9)])
+# nx, ny, nz, npad, planes per segment of the forward and of the backward step on 148
+# SMs (tests/test_sched3d.py computes them)
+GRIDS = [(40, 36, 24, 6, 4, 4), (41, 25, 21, 5, 4, 4), (33, 37, 26, 7, 4, 4), (70, 26, 35, 9, 4, 4),
+         (250, 250, 21, 5, 7, 11), (250, 250, 26, 6, 9, 13), (330, 360, 21, 5, 21, 21)]
+
+
+@pytest.mark.parametrize("nx,ny,nz,npad", [g[:4] for g in GRIDS])
 def test_alternating_march_matches_oracle(ctx, nx, ny, nz, npad):
     s = S.small3d(nx=nx, ny=ny, nz=nz, nt=131, npad=npad, rate=2.8e-3)
     t = S.small3d(nx=nx, ny=ny, nz=nz, nt=131, npad=npad, rate=2.8e-3, seed=11)

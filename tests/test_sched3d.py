@@ -73,3 +73,12 @@ def test_shared_launch_counts_every_volume(scheds):
                 assert len({g[0] for g in got}) == 1  # one depth, one segment length
                 if got[0][0] < 8:
                     assert total <= 148 * ctas
+
+
+def test_segments_of_the_march_test(scheds):
+    """The grids that the GPU test of the march is written for have the segments it
+    names: off the 4-plane blocks, and the whole depth."""
+    from test_gpu_march import GRIDS
+    for per_sm, col in ((3, 4), (2, 5)):
+        got = scheds([(g[0], g[1], g[2], per_sm, 1, 0) for g in GRIDS])
+        assert [s[0] for s in got] == [g[col] for g in GRIDS]
