@@ -12,6 +12,8 @@
 * Bounded waits: a kernel waiting on an mbarrier that nothing completes gives
   up after its poll limit and the host sees VTI_ERR_TIMEOUT through the
   context status word; the context stays usable afterwards.
+* Allocations that fail: the call that asked reports VTI_ERR_OOM, and no later
+  call finds the error again.
 """
 import ctypes as C
 
@@ -145,3 +147,20 @@ def test_bounded_wait_gives_up_and_reports_a_timeout(ctx):
     d = V.modelDataCij3d_f(ctx, s.geom(), s.souloc, [0], s.recloc, s.wavelet, c[:n],
                            c[n:2 * n], c[2 * n:], flags=V.OPT_FULL_STEPS)
     assert np.isfinite(d).all() and np.abs(d).max() > 0
+
+
+def test_a_refused_allocation_is_reported_once(ctx):
+    big = V.geom3d(4000, 4000, 4000, 100, 10, 10.0, 10.0, 10.0, 7e-4, 1.4e-3)  # 256 GB per volume
+    with pytest.raises(V.VtiError) as e:
+        V.Plan3d(ctx, big, V.OPT_FULL_STEPS)
+    assert e.value.status == V.VTI_ERR_OOM
+    s = S.small3d(nx=40, ny=36, nz=32, nt=60, npad=8)
+    n, c = s.nxyz, s.cij()
+    p = V.Plan3d(ctx, s.geom(), V.OPT_FULL_STEPS)
+    try:  # the first launch after the refusal checks for errors
+        p.set_model(c[:n], c[n:2 * n], c[2 * n:])
+        p.set_wavelet(s.wavelet)
+        p.set_receivers(s.recloc)
+        assert np.abs(p.model_data(s.souloc, [0])).max() > 0
+    finally:
+        p.close()

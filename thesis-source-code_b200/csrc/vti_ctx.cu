@@ -15,6 +15,7 @@ int fail(vti_ctx* ctx, int status, const std::string& msg) {
 
 int cuda_check(vti_ctx* ctx, cudaError_t e, const char* what) {
   if (e == cudaSuccess) return VTI_OK;
+  cudaGetLastError();  // reported here; the next launch check must not find it again
   std::string m = std::string(what) + ": " + cudaGetErrorString(e);
   int st = (e == cudaErrorMemoryAllocation) ? VTI_ERR_OOM : VTI_ERR_DEVICE;
   return fail(ctx, st, m);
