@@ -297,9 +297,9 @@ def run_b200(args):
     bwd_avg = bwd_ms / max(bwd_n, 1) / 1e3
     fwd_avg = fwd_ms / max(fwd_n, 1) / 1e3
     achieved = BWD_BYTES_PER_POINT * upd / bwd_avg / 1e9 if bwd_n else None
-    # DRAM bytes per updated point from an ncu capture of in-loop launches on
-    # a smaller grid (traffic grows with the points updated), scaled to this
-    # launch
+    # DRAM bytes per updated point from an ncu capture of in-loop launches at
+    # 400x400x200, scaled to this launch (smaller grids move fewer bytes per
+    # point: a level finds more of the level before in L2)
     traffic = None
     tf = ROOT / "profiles" / "k_bwd3d_tma_traffic.json"
     if tf.exists():
