@@ -186,3 +186,35 @@ def test_nonfinite_samples_spread_as_per_level(ctx, value, nx, nz):
             frame = np.ones((nnz, nnx), bool)
             frame[4:-4, 4:-4] = False
             assert not y[frame].any()
+
+
+def test_calls_of_two_threads_on_one_context(ctx):
+    """Gradients and migrations that two threads run on one context at the same time:
+    only one of them has the context's scratch, the results are those of calls alone."""
+    import threading
+    rng = np.random.default_rng(6)
+    calls = []
+    for nx, nz, pad, nt in ((57, 30, 12, 301), (201, 101, 20, 201)):
+        s = shots(S.survey2d(nx=nx, nz=nz, nt=nt, npad=pad, rate=2e-3), [pad + nx // 2], nx // 3,
+                  pad + 1)
+        data = rng.standard_normal(((nt - 1) // 2 + 1, nx // 3)).astype(np.float32)
+        a = (s.c11, s.c13, s.c33, s.wavelet, s.sloc, s.rloc, s.taper)
+        calls.append(lambda s=s, a=a, data=data: [*V.objFuncGradient_f(ctx, s.geom(), data, *a)[:3],
+                                                  V.rtm_f(ctx, s.geom(), data, *a)])
+    alone = [c() for c in calls]
+    got = [[], []]
+
+    def run(k):
+        for _ in range(8):
+            got[k].append(calls[k]())
+
+    threads = [threading.Thread(target=run, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k in range(2):
+        assert len(got[k]) == 8
+        for out in got[k]:
+            for x, y in zip(out, alone[k]):
+                assert np.abs(y).max() > 0 and np.array_equal(x, y)

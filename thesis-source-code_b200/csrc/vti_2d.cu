@@ -550,11 +550,9 @@ int run2d(vti_ctx* ctx, const vti2d_geom* g, const float* c11, const float* c13,
   const size_t nbuf = 8 * (size_t)nnxz + g->nt;
   const size_t n_ints = (size_t)nrec;
   const size_t n_data = (size_t)nrows_out * nrec;
-  float* buf = nullptr;
-  {
-    const int sst = scratch2d(ctx, (nbuf + n_ints + n_data) * sizeof(float), &buf);
-    if (sst != VTI_OK) return sst;
-  }
+  CallBlock mem;
+  float* buf = mem.get(ctx, (nbuf + n_ints + n_data) * sizeof(float), SIZE_MAX);
+  if (!buf) return fail(ctx, VTI_ERR_OOM, "2D scratch: out of memory");
   float *dc11 = buf, *dc13 = dc11 + nnxz, *dc33 = dc13 + nnxz, *dtap = dc33 + nnxz;
   float* w[4] = {dtap + nnxz, dtap + 2 * nnxz, dtap + 3 * nnxz, dtap + 4 * nnxz};
   float* amps = dtap + 5 * nnxz;
@@ -725,8 +723,9 @@ int synth2d_resident(vti_ctx* ctx, const ResShape& shape, const vti2d_geom* g, c
   for (int ir = 0; ir < nr_total; ++ir) hi.push_back(rloc[2 * ir + 1]);
   const size_t nf = 4 * (size_t)nnxz + g->nt;
   const size_t n_data = (size_t)nrows * nr_total;
-  float* buf = nullptr;
-  VTI_TRY_RES(scratch2d(ctx, (nf + hi.size() + n_data) * sizeof(float), &buf));
+  CallBlock mem;
+  float* buf = mem.get(ctx, (nf + hi.size() + n_data) * sizeof(float), SIZE_MAX);
+  if (!buf) return fail(ctx, VTI_ERR_OOM, "2D scratch: out of memory");
   float *dc11 = buf, *dc13 = dc11 + nnxz, *dc33 = dc13 + nnxz, *dtap = dc33 + nnxz;
   float* amps = dtap + nnxz;
   int* d_ints = reinterpret_cast<int*>(buf + nf);

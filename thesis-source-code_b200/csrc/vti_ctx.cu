@@ -197,36 +197,30 @@ void drop_scratch2d(vti_ctx* ctx) {
 }
 }  // namespace
 
-// The context's 2D scratch, grown (never shrunk) to `bytes`; freed with the
-// context.
-int scratch2d(vti_ctx* ctx, size_t bytes, float** out) {
-  if (ctx->scratch2d_bytes < bytes) {
-    drop_scratch2d(ctx);
-    VTI_CUDA(ctx, cudaMalloc((void**)&ctx->scratch2d, bytes));
-    ctx->scratch2d_bytes = bytes;
-  }
-  *out = ctx->scratch2d;
-  return VTI_OK;
-}
-
-float* CallBlock::get(vti_ctx* ctx, size_t bytes) {
-  if (ctx->scratch2d_bytes >= bytes) return ctx->scratch2d;
-  const bool keep = bytes <= kScratch2dKeep;
-  if (keep) drop_scratch2d(ctx);
+float* CallBlock::get(vti_ctx* ctx, size_t bytes, size_t keep) {
+  hold = std::unique_lock<std::mutex>(ctx->scratch2d_mu, std::try_to_lock);
+  const bool mine = hold.owns_lock();
+  if (mine && ctx->scratch2d_bytes >= bytes) return ctx->scratch2d;
+  const bool grow = mine && bytes <= keep;
+  if (grow) drop_scratch2d(ctx);
   float* p = nullptr;
   if (cudaMalloc((void**)&p, bytes) != cudaSuccess) {
     cudaGetLastError();
-    drop_scratch2d(ctx);
-    if (keep || cudaMalloc((void**)&p, bytes) != cudaSuccess) {
-      cudaGetLastError();
-      return nullptr;
+    p = nullptr;
+    if (mine && !grow) {  // once more without the scratch
+      drop_scratch2d(ctx);
+      if (cudaMalloc((void**)&p, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        p = nullptr;
+      }
     }
   }
-  if (keep) {
+  if (grow && p) {
     ctx->scratch2d = p;
     ctx->scratch2d_bytes = bytes;
   } else {
     own = p;
+    if (mine) hold.unlock();
   }
   return p;
 }

@@ -5,6 +5,7 @@
 #include <nvtx3/nvToolsExt.h>
 #include <cstdint>
 #include <cstdio>
+#include <mutex>
 #include <string>
 #include <utility>
 #include <vector>
@@ -75,6 +76,7 @@ struct vti_ctx {
   // device scratch of the 2D forms, kept between calls
   float* scratch2d = nullptr;
   size_t scratch2d_bytes = 0;
+  std::mutex scratch2d_mu;  // held by the call that uses it
   // staging block of host transfers of pitched volumes, kept between calls
   float* stage = nullptr;
   // plan kept by the one-call 3D forms while their geometry and flags repeat
@@ -160,19 +162,18 @@ int cuda_check(vti_ctx* ctx, cudaError_t e, const char* what);
     if (e_ != cudaSuccess) return ::vti::cuda_check(ctx, e_, what);          \
   } while (0)
 
-// The context's 2D scratch of at least `bytes` bytes (kept between calls, freed
-// with the context).
-int scratch2d(vti_ctx* ctx, size_t bytes, float** out);
-// Device memory of one call of the tiled 2D forms: the context's scratch up to
-// kScratch2dKeep, which a 461 x 261 gradient of 1800 levels reaches (allocating and
-// freeing 590 MB costs 1 to 4 ms of a 6 ms call), beyond that a block of its own,
-// freed with this. get returns null, and leaves no error behind, when the device
-// has no room even without the scratch: the caller then takes the per-level path,
-// which needs less.
+// Device memory of one 2D call: the context's scratch (kept between calls, freed with
+// the context) up to `keep` bytes, beyond that, or while another thread's call on the
+// context has the scratch, a block of its own, freed with this. get returns null,
+// and leaves no error behind, when the device has no room even without the scratch.
+// The tiled forms keep up to kScratch2dKeep, which a 461 x 261 gradient of 1800
+// levels reaches (allocating and freeing 590 MB costs 1 to 4 ms of a 6 ms call), and
+// leave the call to the per-level path, which needs less, when there is no room.
 constexpr size_t kScratch2dKeep = (size_t)1 << 30;
 struct CallBlock {
   float* own = nullptr;
-  float* get(vti_ctx* ctx, size_t bytes);
+  std::unique_lock<std::mutex> hold;  // of the context's scratch
+  float* get(vti_ctx* ctx, size_t bytes, size_t keep = kScratch2dKeep);
   CallBlock() = default;
   CallBlock(const CallBlock&) = delete;
   CallBlock& operator=(const CallBlock&) = delete;
