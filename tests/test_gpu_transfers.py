@@ -81,3 +81,39 @@ def test_product_with_blocks_longer_than_the_record(ctx, nt):
     for o in out[1:]:
         for k in ("hv", "grad", "traces", "born"):
             assert np.array_equal(o[k], out[0][k]), k
+
+
+def test_transfers_of_two_threads_on_one_context(ctx):
+    """Two threads set models and fetch gradients of their own plans on one context:
+    the staging block carries one piece at a time."""
+    import threading
+    plans, models = [], []
+    for k, (nx, ny, nz) in enumerate(((70, 121, 93), (90, 110, 105))):
+        s = S.small3d(nx=nx, ny=ny, nz=nz, nt=12, npad=5, rate=2.1e-3, seed=3 + k)
+        p = V.Plan3d(ctx, s.geom(), V.OPT_FULL_STEPS)
+        p.set_wavelet(s.wavelet)
+        p.set_receivers(s.recloc)
+        dobs = np.random.default_rng(k).standard_normal(
+            V.nnt3d(s.geom()) * (s.recloc.size // 4)).astype(np.float32)
+        plans.append(p)
+        models.append((s.cij().reshape(3, s.nxyz), s.souloc, dobs))
+
+    def call(k):
+        c, sou, dobs = models[k]
+        plans[k].set_model(*c)
+        return plans[k].gradient(sou, [0], dobs)[0]
+
+    alone = [call(0), call(1)]
+    got = [[], []]
+    threads = [threading.Thread(target=lambda k=k: got[k].extend(call(k) for _ in range(40)))
+               for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for p in plans:
+        p.close()
+    for k in range(2):
+        assert len(got[k]) == 40 and np.abs(alone[k][1:]).max() > 0
+        for g in got[k]:
+            assert np.array_equal(g, alone[k])

@@ -114,6 +114,7 @@ __global__ void k_rows(float* flat, float* rows, int nx, int pitch, unsigned n) 
 // The context's staging block for host transfers (kept, freed with the
 // context); null when it cannot be allocated.
 float* stage_block(vti_ctx* ctx) {
+  std::lock_guard<std::mutex> lk(ctx->stage_mu);
   if (!ctx->stage && cudaMalloc((void**)&ctx->stage, kStageBytes) != cudaSuccess) {
     cudaGetLastError();
     ctx->stage = nullptr;
@@ -146,6 +147,9 @@ int host_rows(vti_ctx* ctx, float* dev, int pitch, float* host, int nx, size_t n
   }
   const size_t per = kStageBytes / row;
   for (size_t r = 0; r < nrow; r += per) {
+    // a copy and its kernel follow one another in the stream, whatever other
+    // threads queue there
+    std::lock_guard<std::mutex> lk(ctx->stage_mu);
     const size_t m = std::min(per, nrow - r);
     const unsigned n = (unsigned)(m * nx);
     const int blocks = (int)std::min<unsigned>((n + 255) / 256, 8u * ctx->sm_count);

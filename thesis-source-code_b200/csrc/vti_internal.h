@@ -79,6 +79,7 @@ struct vti_ctx {
   std::mutex scratch2d_mu;  // held by the call that uses it
   // staging block of host transfers of pitched volumes, kept between calls
   float* stage = nullptr;
+  std::mutex stage_mu;  // held while a copy and its kernel are queued
   // plan kept by the one-call 3D forms while their geometry and flags repeat
   bool plan_cache = true;
   vti3d_plan* cached_plan = nullptr;
